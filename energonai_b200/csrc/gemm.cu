@@ -13,6 +13,7 @@
 //       every SM pulls the same number of weight bytes.  A tile shared by several CTAs is
 //       reduced through fp32 partials in a caller-provided workspace by whichever CTA arrives
 //       last, summing in a fixed order, so results are deterministic.
+//   (Few rows against a small weight, where a launch's latency is what counts, take gemm_step.cuh instead.)
 //
 // Warp roles (192 threads): warp 0 = TMA producer (one lane), warp 1 = TMEM allocation and
 // tcgen05.mma issue (one lane), warps 2-5 = epilogue (tcgen05.ld -> bias / activation /
@@ -35,6 +36,7 @@
 
 #include "comm.cuh"
 #include "gated.cuh"
+#include "packed_math.cuh"
 #include "xielu.cuh"
 
 namespace eb {
@@ -1214,6 +1216,7 @@ inline void swap_split(int N, int K, int kpb, int *grid, int *units) {
 constexpr size_t kCounterBytes = 64 * 1024;   // workspace head: four ints per 128-row tile, zero between calls
 
 #include "gemm_chain.cuh"
+#include "gemm_step.cuh"
 
 template <typename T, int BN>
 int launch_chain(const ChainMaps &maps, const ChainParams &p, int grid, size_t smem, cudaStream_t st) {
@@ -1537,6 +1540,14 @@ static int gemm_impl(const void *A, long long lda, const void *W, long long ldw,
     const size_t need = kCounterBytes + (size_t)grid * 2 * bn * kLanes * sizeof(float);
     EB_REQUIRE(workspace && workspace_bytes >= need && aligned16(workspace),
                "gemm: M=%d needs a workspace of %zu bytes, zero-filled once (eb_gemm_workspace_bytes)", M, need);
+    const StepGeometry step = step_geometry(M, K);
+    if (!comm && step_form_pays(M, N, K, step.smem)) {
+#define EB_STEP(NT)                                                       \
+    (dtype == EB_F16 ? launch_step_gemm<__half, NT>(p, W, ldw, step, st)    \
+                     : launch_step_gemm<__nv_bfloat16, NT>(p, W, ldw, step, st))
+      return M <= 8 ? EB_STEP(1) : M <= 16 ? EB_STEP(2) : EB_STEP(4);
+#undef EB_STEP
+    }
     p.counters = reinterpret_cast<int *>(workspace);
     p.partial = reinterpret_cast<float *>(reinterpret_cast<char *>(workspace) + kCounterBytes);
     p.lane_rows = N; p.col_rows = M;

@@ -187,3 +187,44 @@ def test_gemm_ln_fold_rejects_wide_batches():
     w_f, colsum, bias32 = fold_layernorm(w, None, ones, ones)
     with pytest.raises(RuntimeError):
         gemm(x, w_f, ln_fold=(colsum, bias32, 1e-5))
+
+
+# Few rows against small weights (one CTA per 16 weight rows, its warps splitting K): batch rows around the
+# multiples of 8, K below one slice, with an empty last slice and not a multiple of 32, N not a multiple of 16, more
+# tiles than CTAs, and both sides of the sizes up to which that form is taken.
+STEP_SHAPES = [(1, 8, 8), (7, 40, 40), (8, 5000, 264), (9, 768, 776), (16, 24, 3072), (17, 1000, 2056), (32, 520, 520), (31, 2048, 2048), (32, 2056, 2048),
+               (1, 16392, 4096), (8, 4104, 4096), (16, 2048, 4096), (16, 4112, 2048), (3, 50257, 64)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K", STEP_SHAPES)
+def test_gemm_few_rows(M, N, K, dtype):
+    """Every epilogue; the folded LayerNorm with a row mean of several standard deviations (its single-pass sums are
+    fp32: 1e-5 of the row maximum, as REL has it, and the mean times the column sum on top, hence 1e-4)."""
+    from energonai_b200.gemm import fold_layernorm, gemm, gemm_parts, project_unit
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N * 3 + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, w, b, res = rnd(M, K).to(dtype), (rnd(N, K) * K ** -0.5).to(dtype), rnd(N).to(dtype), rnd(M, N).to(dtype)
+    plain = reference(x, w)
+    check_close(gemm(x, w, bias=b, act="relu", residual=res, static_weight=True), reference(x, w, b, "relu", res), dtype)
+    check_close(gemm(x, w, bias=b, out_dtype=torch.float32), plain + b.float(), torch.float32)
+    # one row of a cache, its number on the device; nothing else is written, and nothing at all beyond the limit
+    cache, row = torch.zeros(M, 3, N + 8, device="cuda", dtype=dtype), torch.tensor([1], dtype=torch.int32, device="cuda")
+    where = dict(out=cache, out_rows_per_batch=1, out_batch_stride=cache.stride(0), out_ld=cache.stride(1), out_row_offset_device=row)
+    gemm(x, w, out_row_limit=3, **where)
+    check_close(cache[:, 1, :N], plain, dtype)
+    assert not cache[:, [0, 2]].any() and not cache[:, 1, N:].any()
+    status_ok()
+    if N % 16 == 0:
+        gate, up = plain.view(M, N // 16, 2, 8).unbind(2)
+        check_close(project_unit(x, w, "geglu"), (torch.nn.functional.gelu(gate, approximate="tanh") * up).reshape(M, N // 2), dtype)
+    if N % 8 == 0 and N > 16:
+        out, tail = gemm_parts(x, w, bias=b, tail_col=N - 8)
+        check_close(out, (plain + b.float())[:, :N - 8], dtype)
+        check_close(tail, (plain + b.float())[:, N - 8:], torch.float32)
+    shifted, gamma, beta = (x.float() + 3).to(dtype), (torch.rand(K, device="cuda", generator=g) + 0.5).to(dtype), rnd(K).to(dtype)
+    folded, colsum, bias32 = fold_layernorm(w, b, gamma, beta)
+    got = gemm(shifted, folded, ln_fold=(colsum, bias32, 1e-5), out_dtype=torch.float32, static_weight=True)
+    want = torch.nn.functional.layer_norm(shifted.double(), (K,)) @ folded.double().t() + bias32.double()
+    assert float((got - want).abs().max()) < 1e-4 * float(want.abs().max())
+    status_ok()
