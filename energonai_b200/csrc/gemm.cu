@@ -13,7 +13,7 @@
 //       every SM pulls the same number of weight bytes.  A tile shared by several CTAs is
 //       reduced through fp32 partials in a caller-provided workspace by whichever CTA arrives
 //       last, summing in a fixed order, so results are deterministic.
-//   (Few rows against a small weight, where a launch's latency is what counts, take gemm_step.cuh instead.)
+//   (Prompt-sized products take a tile of 256 rows per pair of SMs, gemm_pair.cuh, where that is faster.  Few rows against a small weight, where a launch's latency is what counts, take gemm_step.cuh instead.)
 //
 // Warp roles (192 threads): warp 0 = TMA producer (one lane), warp 1 = TMEM allocation and
 // tcgen05.mma issue (one lane), warps 2-5 = epilogue (tcgen05.ld -> bias / activation /
@@ -1118,6 +1118,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tm_lane, const __grid_constant__
   }
 }
 
+#include "gemm_pair.cuh"
+
 // ---- host side --------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -1182,6 +1184,23 @@ int launch(const CUtensorMap &tl, const CUtensorMap &tc, const GemmParams &p, in
     configured[dev] = 227 * 1024;
   }
   launch_pdl(kern, dim3(grid), dim3(kThreads), smem, st, tl, tc, p);
+  return check_launch("gemm");
+}
+
+template <typename T, int BN, int EW>
+int launch_pair(const CUtensorMap &ta, const CUtensorMap &tw, const GemmParams &p, int grid, size_t smem, cudaStream_t st) {
+  auto kern = gemm_pair_kernel<T, BN, EW>;
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(EB_ECUDA, "gemm: cannot reserve shared memory");
+    }
+    configured[dev] = true;
+  }
+  launch_pdl(kern, dim3(grid), dim3(64 + 32 * EW), smem, st, ta, tw, p);
   return check_launch("gemm");
 }
 
@@ -1569,27 +1588,48 @@ static int gemm_impl(const void *A, long long lda, const void *W, long long ldw,
   }
   p.lane_rows = M; p.col_rows = N;
   const long long lane_tiles = (M + kLanes - 1) / kLanes;
-  // Tile width: a k-block costs a CTA about 0.45 / 0.30 / 0.23 / 0.19 us with 256 / 128 / 64 / 32 columns (2, 2 and 3 k-blocks
-  // per stage for the narrow ones, whose pace is the hand-over of a stage), and the tiles come in waves of one per
-  // SM.  What a row's result is does not depend on the choice.
-  struct Form { int bn, kpb, stages; float us; };
-  constexpr Form forms[] = {{256, 1, 4, 0.45f}, {128, 2, 3, 0.30f}, {64, 2, 4, 0.23f}, {32, 3, 3, 0.19f}};
-  auto waves = [&](int cols) { return (lane_tiles * ((N + cols - 1) / cols) + sm_count() - 1) / sm_count(); };
-  Form form = forms[0];
+  // Form: the tiles come in waves of one per SM (or pair of SMs); a wave costs its k-blocks and, at its end, an epilogue.  Measured on
+  // products of 64 to 16384 rows, 768 to 20480 columns and K 768 to 20480, microseconds: {columns, one-SM: k-blocks per stage, stages, per
+  // k-block, per wave}; the choice is within 10 % of the best form at all of them.  The narrow pair tile is bound by L2 once most SMs
+  // stay busy (0.27).  One-SM tiles stay for few rows (128 x 4096 x 4096: 32 columns 14.0 us, best pair 17.1; 333 x 5120 x 5120: 128 columns
+  // 26.0 against 32.4) and lose elsewhere: 8192 x 5120 x 5120 391 us against 299, 12448 x 1024 x 1024 40 against 27, 1024 x 2304 x 768 10.9
+  // against 9.1.  What a row's result is does not depend on the choice.
+  struct Form { int rows, bn, kpb, stages; float us, wave; };
+  constexpr Form forms[] = {{256, 256, 2, 3, 0.37f, 3.6f}, {256, 128, 2, 4, 0.20f, 1.6f}, {128, 256, 1, 4, 0.45f, 6.f},
+                            {128, 128, 2, 3, 0.28f, 3.2f}, {128, 64, 2, 4, 0.20f, 1.8f},  {128, 32, 3, 3, 0.14f, 1.f}};
+  Form form = forms[2];
+  long long waves = 0;
   if (p.rs) {                                          // (its epilogue turns 64 columns around behind 1-block stages)
-    if (lane_tiles * ((N + 255) / 256) < sm_count()) form = {128, 1, 6, 0.f};
+    if (lane_tiles * ((N + 255) / 256) < sm_count()) form = {128, 128, 1, 6, 0.f, 0.f};
   } else {
     float best = 0.f;
     for (const Form &f : forms) {
-      const float us = (float)waves(f.bn) * ((float)p.kblocks * f.us + 2.f);
-      if (f.bn == 256 || us < best) { best = us; form = f; }
+      const long long units = sm_count() * 128 / f.rows, w = ((long long)((M + f.rows - 1) / f.rows) * ((N + f.bn - 1) / f.bn) + units - 1) / units;
+      const float us = (float)w * ((float)p.kblocks * (f.rows == 256 && f.bn == 128 && w > 3 ? 0.27f : f.us) + f.wave);
+      if (waves == 0 || us < best) { best = us; form = f; waves = w; }
     }
+  }
+  p.kpb = form.kpb;
+  p.stages = form.stages;
+  if (form.rows == 256) {
+    const int bn = form.bn;
+    const long long tiles = (long long)((M + 255) / 256) * ((N + bn - 1) / bn), pairs = sm_count() / 2;
+    const int grid = 2 * (int)(tiles < pairs ? tiles : pairs);
+    const size_t smem = kBarrierBytes + 1024 + (size_t)p.stages * kPairBlocks * (kLanes * 128 + bn / 2 * 128) + 16 * kPairStagingBytes;
+    if ((rc = make_map(&tl, A, dtype, M, K, lda, kLanes))) return rc;
+    if ((rc = make_map(&tc, W, dtype, N, K, ldw, bn / 2))) return rc;
+#define EB_PAIR(BN, EW)                                                                  \
+  (dtype == EB_F16 ? launch_pair<__half, BN, EW>(tl, tc, p, grid, smem, st)              \
+                   : launch_pair<__nv_bfloat16, BN, EW>(tl, tc, p, grid, smem, st))
+    // Sixteen epilogue warps where the epilogue is what a wave ends with or, at a short K, what it lasts (12448 x 4096 x 1024 with erf-GELU:
+    // 111 us against 146 with eight, 1024 x 768 x 768 10.8 against 12.6); eight disturb a long main loop less (8192 x 5120 x 5120: 299 against 358).
+    if (bn == 128) return EB_PAIR(128, 16);
+    return K <= 2048 || waves <= 2 ? EB_PAIR(256, 16) : EB_PAIR(256, 8);
+#undef EB_PAIR
   }
   const int bn = form.bn;
   const long long tiles = lane_tiles * ((N + bn - 1) / bn);
   const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-  p.kpb = form.kpb;
-  p.stages = form.stages;
   // (+ 18 KB behind the stages: the staging rows of the reduce-scatter epilogue)
   const size_t smem = kBarrierBytes + 1024 + (size_t)p.stages * p.kpb * (kLanes * 128 + bn * 128) + (p.rs ? 4 * 32 * 72 * 2 : 0);
   if ((rc = make_map(&tl, A, dtype, M, K, lda, kLanes))) return rc;

@@ -228,3 +228,39 @@ def test_gemm_few_rows(M, N, K, dtype):
     want = torch.nn.functional.layer_norm(shifted.double(), (K,)) @ folded.double().t() + bias32.double()
     assert float((got - want).abs().max()) < 1e-4 * float(want.abs().max())
     status_ok()
+
+
+# Tiles of 256 rows per pair of SMs: narrow and wide, few and many waves (16 and 8 epilogue warps); a last row tile of one row and with an
+# empty second half, N ending inside a tile and a chunk, K below a k-block, with an odd number of k-blocks and not a multiple of 64.
+PAIR_SHAPES = [(257, 8200, 72), (513, 2056, 776), (5000, 4112, 8), (700, 3088, 840), (6000, 2064, 136), (2300, 4112, 2120)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,N,K", PAIR_SHAPES)
+def test_gemm_pair_tiles(M, N, K, dtype):
+    from energonai_b200.gemm import gemm, gemm_parts, project_unit
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N * 3 + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, w, b, res = rnd(M, K).to(dtype), (rnd(N, K) * K ** -0.5).to(dtype), rnd(N).to(dtype), rnd(M, N).to(dtype)
+    plain = reference(x, w)
+    for act in ("relu", "gelu", "gelu_tanh"):
+        check_close(gemm(x, w, bias=b, act=act), reference(x, w, b, act), dtype)
+    # the result in place of the residual, as the blocks have it
+    got = res.clone()
+    gemm(x, w, bias=b, residual=got, out=got, static_weight=True)
+    check_close(got, reference(x, w, b, None, res), dtype)
+    check_close(gemm(x, w, bias=b, out_dtype=torch.float32), plain + b.float(), torch.float32)
+    # batch rows of a cache, from a row on whose number is on the device; nothing else is written, and nothing at all beyond the limit
+    batch = next(d for d in (4, 3, 2, 1) if M % d == 0)
+    cache, row = torch.zeros(batch, M // batch + 2, N + 8, device="cuda", dtype=dtype), torch.tensor([1], dtype=torch.int32, device="cuda")
+    gemm(x, w, out=cache, out_rows_per_batch=M // batch, out_batch_stride=cache.stride(0), out_ld=cache.stride(1), out_row_offset_device=row, out_row_limit=2)
+    check_close(cache[:, 1:-1, :N].reshape(M, N), plain, dtype)
+    assert not cache[:, [0, -1]].any() and not cache[:, :, N:].any()
+    status_ok()
+    if N % 16 == 0:
+        gate, up = plain.view(M, N // 16, 2, 8).unbind(2)
+        check_close(project_unit(x, w, "geglu"), (torch.nn.functional.gelu(gate, approximate="tanh") * up).reshape(M, N // 2), dtype)
+    out, tail = gemm_parts(x, w, bias=b, tail_col=N - 24)
+    check_close(out, (plain + b.float())[:, :N - 24], dtype)
+    check_close(tail, (plain + b.float())[:, N - 24:], torch.float32)
+    status_ok()
