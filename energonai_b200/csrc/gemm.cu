@@ -1413,6 +1413,7 @@ int attention_tc_status(int *out4, bool clear);   // attention_tc.cu
 int latent_status(int *out4, bool clear);         // latent_attention.cu
 int memory_tc_status(int *out4, bool clear);      // matrix_memory_tc.cu
 int decay_tc_status(int *out4, bool clear);       // decay_memory_tc.cu
+int f32_status(int *out4, bool clear);            // gemm_f32.cu
 }
 
 extern "C" int eb_device_status(int *out4, int clear) {
@@ -1449,6 +1450,12 @@ extern "C" int eb_device_status(int *out4, int clear) {
   if (host[0] == 0 && dec[0] != 0) {
     for (int i = 0; i < 4; ++i) host[i] = dec[i];
     host[1] += 400;
+  }
+  int f32[4] = {0, 0, 0, 0};                       // fp32 products: 500+
+  if (eb::f32_status(f32, clear != 0) != EB_OK) return fail(EB_ECUDA, "device_status: cannot read the status word");
+  if (host[0] == 0 && f32[0] != 0) {
+    for (int i = 0; i < 4; ++i) host[i] = f32[i];
+    host[1] += 500;
   }
   if (out4)
     for (int i = 0; i < 4; ++i) out4[i] = host[i];

@@ -1,11 +1,12 @@
-// C = A . W^T with fp32 operands and plain fp32 multiply-adds (no reduced-precision tensor mode):
-// the product of models that are run in true 32-bit.  A tiled CUDA-core kernel, 64 x 64 outputs per
-// CTA.  Groups, two ways:
+// C = A . W^T with fp32 operands to fp32 precision: the product of models that are run in true 32-bit.  Groups, two ways:
 //   tile_group != null   the rows of A come in 128-row tiles, tile i using the weights of group
 //                        tile_group[i]; tiles from *live_tiles on are skipped
 //   groups > 1           blockIdx.z = group: strides between the groups' operands
-// A single product may add a bias and apply xIELU to its first columns.
+// A single product may add a bias and apply xIELU to its first columns.  Two kernels:
+//   gemm_f32_tc_kernel   tensor cores, every operand split into three bf16 pieces
+//   gemm_f32_kernel      what it does not take: operands that 16-byte loads cannot read, a K below 64
 #include "common.cuh"
+#include "tc_ops.cuh"
 #include "xielu.cuh"
 
 namespace eb {
@@ -23,6 +24,205 @@ struct F32Params {
   int act_cols;
 };
 
+// ---- tensor cores -------------------------------------------------------------------------------------------------
+// A CTA computes 128 rows of A x 64 rows of W.  An fp32 number is the sum of three bf16 numbers (rounded, and twice the exact
+// remainder rounded); of the nine products of pieces the three smallest, below 2^-25 of the whole and of either sign, are left out.
+// Per chunk of 64 columns six products of 128 x 64 x 64 go to the tensor core, the smallest first, into an accumulator that starts at zero;
+// four warps add the finished chunk to sums in registers.  The tensor core truncates when it accumulates (a K of 2048 summed there is off
+// by 2e-6 and too small on average, one of 4096 by 4e-6); over one chunk that is 7e-8, and the whole is closer to 64-bit results than a
+// chain of fp32 multiply-adds: K = 64 7.7e-8 against 1.4e-7, K = 2048 1.3e-7 against 8.1e-7, K = 5632 1.9e-7 against 1.3e-6 (2-norm, normal operands).
+// Bound by the trip to L2 for a chunk's operands, of which one chunk is requested ahead (48 registers a thread), and by splitting them.
+// Warps 0-3 add up and store, 4-11 load, split and write the swizzled operand tiles, 12 issues the products.
+// An infinity, a NaN or a number that bf16 rounds to infinity has no such split: the outputs of its row are computed again by
+// multiply-adds.
+constexpr int kF32Cols = 64, kF32Chunk = 64, kSplitWarps = 8, kF32TcThreads = 32 * (4 + kSplitWarps + 1), kF32Stages = 3;
+constexpr uint32_t kPlaneA = kRows * 128, kPlaneW = kF32Cols * 128, kF32StageBytes = 3 * (kPlaneA + kPlaneW);
+constexpr size_t kF32TcSmem = 1024 + 1024 + (size_t)kF32Stages * kF32StageBytes;
+
+// Pieces of two numbers, packed: hi, mid, lo.  Returns the magnitude bits of lo, at least 0x7f80 in a half whose number has no split.
+__device__ __forceinline__ uint32_t round2(float x0, float x1) {
+  uint32_t v;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(x1), "f"(x0));
+  return v;
+}
+__device__ __forceinline__ uint32_t split2(float x0, float x1, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
+  hi = round2(x0, x1);
+  x0 -= __uint_as_float(hi << 16); x1 -= __uint_as_float(hi & 0xffff0000u);
+  mid = round2(x0, x1);
+  lo = round2(x0 - __uint_as_float(mid << 16), x1 - __uint_as_float(mid & 0xffff0000u));
+  return lo & 0x7fff7fffu;
+}
+
+__device__ __forceinline__ void store_f32(const F32Params &p, float *C, int m, int n, float v, float up, float down) {
+  v += p.bias ? p.bias[n] : 0.f;
+  if (p.act_params && n < p.act_cols) v = xielu_exact(v, up, down);
+  C[(long long)m * p.ldc + n] = v;
+}
+
+__global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_addr = s32(smem_raw);
+  uint8_t *smem = smem_raw + (((raw_addr + 1023u) & ~1023u) - raw_addr);
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
+  const uint32_t full = s32(bars), empty = full + 8 * kF32Stages, tfull = empty + 8 * kF32Stages, tempty = tfull + 16;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kF32Stages + 4);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  volatile uint8_t *odd = smem + 512;                  // per row of A, then of W: holds a number that cannot be split
+  const uint32_t tiles = s32(smem) + 1024;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.y * kRows, n0 = blockIdx.x * kF32Cols, chunks = (p.K + kF32Chunk - 1) / kF32Chunk;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kF32Stages; ++s) { bar_init(full + 8 * s, kSplitWarps); bar_init(empty + 8 * s, 1); }
+    for (int a = 0; a < 2; ++a) { bar_init(tfull + 8 * a, 1); bar_init(tempty + 8 * a, 4); }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (threadIdx.x < kRows + kF32Cols) odd[threadIdx.x] = 0;
+  if (warp == 12) {
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(2u * kF32Cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  griddep_wait();
+  griddep_launch();
+  long long group = blockIdx.z;
+  bool live = true;
+  if (p.tile_group) {
+    live = (int)blockIdx.y < *p.live_tiles;
+    group = live ? p.tile_group[blockIdx.y] : 0;
+  }
+  const float *A = p.A + (p.tile_group ? 0 : group * p.a_gs), *W = p.W + group * p.w_gs;
+  float *C = p.C + (p.tile_group ? 0 : group * p.c_gs);
+  float acc[kF32Cols];
+
+  if (!live) {
+  } else if (warp < 4) {
+    // ---------------- sums of the chunks: a thread has a row ----------------
+#pragma unroll
+    for (int j = 0; j < kF32Cols; ++j) acc[j] = 0.f;
+    for (int c = 0; c < chunks; ++c) {
+      const int b = c & 1;
+      if (!__all_sync(0xffffffffu, bar_wait(tfull + 8 * b, (c >> 1) & 1, abort_flag, 1))) break;
+      tc_fence_after();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float v[32];
+        tc_ld32(tmem + ((uint32_t)(warp * 32) << 16) + b * kF32Cols + h * 32, v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[h * 32 + j] += v[j];
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) bar_arrive(tempty + 8 * b);
+    }
+  } else if (warp < 12) {
+    // ---------------- loads and splits: eight threads per row, 8 columns each ----------------
+    constexpr int kPasses = (kRows + kF32Cols) / 32;
+    const int t = threadIdx.x - 128, unit = t & 7, row_in = t >> 3;
+    float4 x[kPasses][2];
+    auto load = [&](int q, int c) {
+      const int row = q * 32 + row_in, k = c * kF32Chunk + unit * 8;
+      const bool of_a = q < kRows / 32;
+      const int r = of_a ? m0 + row : n0 + row - kRows;
+      const bool ok = r < (of_a ? p.M : p.N);
+      const float *src = (of_a ? A + (long long)r * p.lda : W + (long long)r * p.ldw) + k;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        x[q][h] = ok && k + 4 * h < p.K ? __ldg(reinterpret_cast<const float4 *>(src) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+#pragma unroll
+    for (int q = 0; q < kPasses; ++q) load(q, 0);
+    int stage = 0;
+    uint32_t phase = 0, bad = 0;
+    for (int c = 0; c < chunks; ++c) {
+      if (!__all_sync(0xffffffffu, bar_wait(empty + 8 * stage, phase ^ 1u, abort_flag, 2))) break;
+      uint8_t *at = smem + 1024 + (size_t)stage * kF32StageBytes;
+#pragma unroll
+      for (int q = 0; q < kPasses; ++q) {
+        const bool of_a = q < kRows / 32;
+        const int row = (of_a ? q : q - kRows / 32) * 32 + row_in;
+        uint8_t *dst = at + (of_a ? 0 : 3 * kPlaneA) + row * 128 + ((unit ^ (row & 7)) << 4);
+        const uint32_t plane = of_a ? kPlaneA : kPlaneW;
+        uint4 hi, mid, lo;
+        uint32_t worst = __vmaxu2(split2(x[q][0].x, x[q][0].y, hi.x, mid.x, lo.x), split2(x[q][0].z, x[q][0].w, hi.y, mid.y, lo.y));
+        worst = __vmaxu2(worst, split2(x[q][1].x, x[q][1].y, hi.z, mid.z, lo.z));
+        worst = __vmaxu2(worst, split2(x[q][1].z, x[q][1].w, hi.w, mid.w, lo.w));
+        bad |= (worst + 0x00800080u) & 0x80008000u ? 1u << q : 0u;             // (a half of 0x7f80 or more)
+        *reinterpret_cast<uint4 *>(dst) = hi;
+        *reinterpret_cast<uint4 *>(dst + plane) = mid;
+        *reinterpret_cast<uint4 *>(dst + 2 * plane) = lo;
+        if (c + 1 < chunks) load(q, c + 1);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) bar_arrive(full + 8 * stage);
+      if (++stage == kF32Stages) { stage = 0; phase ^= 1u; }
+    }
+    for (int q = 0; q < kPasses; ++q)
+      if (bad >> q & 1u) odd[q * 32 + row_in] = 1;
+  } else {
+    // ---------------- products ----------------
+    constexpr uint32_t idesc = tc_idesc(kF32Cols, 1);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int c = 0; c < chunks; ++c) {
+      const int b = c & 1;
+      if (!__all_sync(0xffffffffu, bar_wait(tempty + 8 * b, ((c >> 1) & 1) ^ 1u, abort_flag, 3))) break;
+      if (!__all_sync(0xffffffffu, bar_wait(full + 8 * stage, phase, abort_flag, 4))) break;
+      tc_fence_after();
+      const uint32_t at = tiles + stage * kF32StageBytes, wt = at + 3 * kPlaneA, d = tmem + b * kF32Cols;
+      // (piece of A, piece of W), smallest products first
+      constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pw[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        const uint64_t da = tc_desc(at + pa[i] * kPlaneA), dw = tc_desc(wt + pw[i] * kPlaneW);
+#pragma unroll
+        for (int k = 0; k < kF32Chunk / 16; ++k) tc_mma_warp(d, da + 2 * k, dw + 2 * k, idesc, i > 0 || k > 0 ? 1u : 0u);
+      }
+      tc_commit_warp(empty + 8 * stage);
+      tc_commit_warp(tfull + 8 * b);
+      if (++stage == kF32Stages) { stage = 0; phase ^= 1u; }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 12) {
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * kF32Cols) : "memory");
+  }
+  if (!live || warp >= 4 || *abort_flag) return;
+  const int m = m0 + warp * 32 + lane;
+  if (m >= p.M) return;
+#pragma unroll
+  for (int j = 0; j < kF32Cols; ++j) {
+    if (!(odd[warp * 32 + lane] | odd[kRows + j]) || n0 + j >= p.N) continue;
+    float v = 0.f;
+    for (int k = 0; k < p.K; ++k) v = fmaf(A[(long long)m * p.lda + k], W[(long long)(n0 + j) * p.ldw + k], v);
+    acc[j] = v;
+  }
+  float up = 0.f, down = 0.f;
+  if (p.act_params) { up = p.act_params[0]; down = p.act_params[1]; }
+  const bool wide = !p.bias && !p.act_params && ((uintptr_t)C & 15) == 0 && p.ldc % 4 == 0;
+#pragma unroll
+  for (int j = 0; j < kF32Cols; j += 4) {
+    if (wide && n0 + j + 4 <= p.N) {
+      *reinterpret_cast<float4 *>(C + (long long)m * p.ldc + n0 + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (n0 + j + e < p.N) store_f32(p, C, m, n0 + j + e, acc[j + e], up, down);
+    }
+  }
+}
+
+// ---- any operands: a tiled CUDA-core kernel, 64 x 64 outputs per CTA ----------------------------------------------------------------
 __global__ void __launch_bounds__(kF32Threads) gemm_f32_kernel(const F32Params p) {
   __shared__ float sa[kStep][kT + 4], sw[kStep][kT + 4];
   griddep_wait();
@@ -66,13 +266,15 @@ __global__ void __launch_bounds__(kF32Threads) gemm_f32_kernel(const F32Params p
     for (int j = 0; j < 4; ++j) {
       const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
       if (m >= p.M || n >= p.N) continue;
-      float v = acc[i][j] + (p.bias ? p.bias[n] : 0.f);
-      if (p.act_params && n < p.act_cols) v = xielu_exact(v, up, down);
-      C[(long long)m * p.ldc + n] = v;
+      store_f32(p, C, m, n, acc[i][j], up, down);
     }
 }
 
 }  // namespace
+
+// Status words of this file's kernels, for eb_device_status.
+int f32_status(int *out4, bool clear) { return tc_status(out4, clear); }
+
 }  // namespace eb
 
 using namespace eb;
@@ -92,6 +294,25 @@ extern "C" int eb_gemm_f32(const float *A, long long lda, long long a_group_stri
   p.A = A; p.W = W; p.C = C; p.lda = lda; p.ldw = ldw; p.ldc = ldc; p.a_gs = a_group_stride; p.w_gs = w_group_stride; p.c_gs = c_group_stride;
   p.M = M; p.N = N; p.K = K; p.tile_group = tile_group; p.live_tiles = live_tiles;
   p.bias = bias; p.act_cols = act_cols; p.act_params = act_params;
-  launch_pdl(gemm_f32_kernel, dim3((N + kT - 1) / kT, (M + kT - 1) / kT, groups), dim3(kF32Threads), 0, as_stream(stream), p);
+  cudaStream_t st = as_stream(stream);
+  // 16-byte loads need rows that begin and end on 16 bytes, and below a chunk the multiply-adds are the closer ones (K = 4: 4.0e-8 against
+  // 4.6e-8).  However many rows there are: a row's result is the same in every batch.  333 x 11264 x 2048: 881 us by multiply-adds, 195 so; one
+  // row x 2048 x 2048 151 and 43.
+  const bool packs = K >= kF32Chunk && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && a_group_stride % 4 == 0 && w_group_stride % 4 == 0 && aligned16(A) && aligned16(W);
+  if (packs) {
+    static bool configured[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev >= 0 && dev < 64 && !configured[dev]) {
+      if (cudaFuncSetAttribute(gemm_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kF32TcSmem) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(EB_ECUDA, "gemm_f32: cannot reserve shared memory");
+      }
+      configured[dev] = true;
+    }
+    launch_pdl(gemm_f32_tc_kernel, dim3((N + kF32Cols - 1) / kF32Cols, (M + kRows - 1) / kRows, groups), dim3(kF32TcThreads), kF32TcSmem, st, p);
+    return check_launch("gemm_f32");
+  }
+  launch_pdl(gemm_f32_kernel, dim3((N + kT - 1) / kT, (M + kT - 1) / kT, groups), dim3(kF32Threads), 0, st, p);
   return check_launch("gemm_f32");
 }

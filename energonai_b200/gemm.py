@@ -120,7 +120,7 @@ def xielu_params(p, q):
 
 
 def gemm_f32(a, w, bias=None, xielu=None):
-    """a [M,K] @ w [N,K].T (+ bias) in true 32-bit (CUDA cores, no reduced-precision mode); xielu =
+    """a [M,K] @ w [N,K].T (+ bias) to 32-bit precision (no reduced-precision mode); xielu =
     (act_params, act_cols) as in gemm_parts."""
     act_params, act_cols = xielu if xielu is not None else (None, 0)
     require_cuda(a, w, bias, act_params)

@@ -273,3 +273,33 @@ def test_latent_decode(R, H, rows, window, pos):
 def test_no_wait_ran_out():
     from energonai_b200.gemm import device_status
     assert device_status()[0] == 0
+
+
+# Tensor cores from K = 64 on: one row and a tile and a row, columns and K around their chunks of 64, bias, many products side by side.  Six products of
+# bf16 pieces leave out 2^-25 of each term; a chunk's sum is truncated to 2^-24 a few times and the chunks are added in fp32.
+@pytest.mark.parametrize("M,N,K", [(1, 9, 64), (33, 63, 68), (128, 64, 128), (129, 65, 132), (257, 200, 2052)])
+def test_gemm_f32_by_pieces(M, N, K):
+    from energonai_b200.gemm import device_status, gemm_f32
+    from energonai_b200.moe import per_head
+    a, w, b = rnd(M, K, dtype=F32), rnd(N, K, seed=1, scale=K ** -0.5, dtype=F32), rnd(N, seed=2, dtype=F32)
+    want = a.double().cpu() @ w.double().cpu().T
+    error = lambda y: float((y.double().cpu() - want).norm() / want.norm())
+    got = gemm_f32(a, w)
+    padded = torch.zeros(M, K + 1, device="cuda")                   # rows that 16-byte loads cannot read: multiply-adds
+    padded[:, :K] = a
+    assert error(got) < 2.5e-7 and error(got) <= error(gemm_f32(padded[:, :K], w)) + 2 ** -24
+    assert torch.equal(gemm_f32(a[-1:], w), got[-1:])               # independent of the batch, bit for bit
+    close(gemm_f32(a, w, bias=b), want + b.double().cpu(), 1e-6)
+    heads = per_head(a.repeat(1, 3), torch.stack([w, 2 * w, -w]))
+    assert torch.equal(heads.view(M, 3, N), torch.stack([got, 2 * got, -got], 1))
+    # what has no pieces: the rows and columns that hold it as multiply-adds have them, all others as before
+    a2, w2 = a.clone(), w.clone()
+    a2[0, K - 1], w2[N - 1, 0] = float("inf"), float("nan")
+    a2[M - 1, 1] = 3.4e38                                           # (rounds to infinity in bf16)
+    got2, plain = gemm_f32(a2, w2), a2.double().cpu() @ w2.double().cpu().T
+    assert torch.equal(got2[1:M - 1, :N - 1], got[1:M - 1, :N - 1])
+    assert torch.equal(got2.isnan().cpu(), plain.isnan()) and got2[:, N - 1].isnan().all()
+    assert (got2[0, :N - 1].cpu() == plain[0, :N - 1].float()).all()
+    if M > 1 and N > 1:
+        close(got2[M - 1, :N - 1] / 3e38, plain[M - 1, :N - 1] / 3e38, 1e-6)
+    assert device_status()[0] == 0
