@@ -8,7 +8,7 @@
 //                    on mma.sync with fp32 scores, statistics and accumulators, cache tiles by TMA.
 //                    The key range is split over the CTAs of a cluster, which merge their parts
 //                    through distributed shared memory (or over more CTAs and a merge kernel).
-//   attention_plain  any head sizes, fp32 or 16 bit, one warp per query row: the path of models run
+//   attention_plain  any head sizes, fp32 or 16 bit, one warp per query row (prompts: tiles of 32 rows): the path of models run
 //                    in 32-bit and of head sizes the tensor-core kernels do not have.
 //
 // Keys are addressed by position: the cache row of position j is j mod ring_rows (a cache that holds
@@ -672,7 +672,139 @@ __global__ void attention_plain_kernel(const PlainParams p) {
   for (int d = lane; d < p.dv; d += 32) o[d] = from_f32<T>(so[d] * inv);
 }
 
+// The same for prompts: a CTA takes 32 rows of a head (four per warp) and walks the positions its rows see 32 at a time, their keys and values
+// in shared memory as fp32.  A warp by itself read every key row on its own, 4 bytes of 32 rows per load: 333 rows of 16 to 32 heads of 64 to 128
+// columns took 1080 us, 185 so.  In the products a lane has a key (scores: 16 bytes of it against four rows' queries) or columns of the output.
+constexpr int kTiledWarps = 8, kTiledRows = 4, kTiledKeys = 32, kTiledWidth = 128;
+
+inline size_t tiled_smem(int dk, int dv) {
+  return sizeof(float) * ((size_t)kTiledKeys * (dk + 4) + (size_t)kTiledKeys * dv + (size_t)kTiledWarps * kTiledRows * (dk + kTiledKeys));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTiledWarps * 32) attention_tiled_kernel(const PlainParams p) {
+  extern __shared__ __align__(16) float pl_smem[];
+  griddep_wait();
+  griddep_launch();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, h = blockIdx.y, b = blockIdx.z;
+  const int kp = p.dk + 4;                               // (a multiple of 4, and 4 mod 32 words apart: no bank conflicts)
+  float *sk = pl_smem, *sq = sk + kTiledKeys * kp + warp * kTiledRows * p.dk, *sp = sk + kTiledKeys * kp + kTiledWarps * kTiledRows * p.dk + warp * kTiledKeys * kTiledRows;
+  float *sv = sk + kTiledKeys * kp + kTiledWarps * kTiledRows * (p.dk + kTiledKeys);
+  const int i0 = blockIdx.x * kTiledWarps * kTiledRows, base = p.pos_dev ? *p.pos_dev : 0, first = p.first ? p.first[b] : 0;
+  auto lowest = [&](int pos) {
+    int lo = first;
+    if (p.window > 0) lo = max(lo, pos - p.window + 1);
+    if (p.chunk > 0 && pos > lo) lo += (pos - lo) / p.chunk * p.chunk;
+    return max(lo, max(0, pos - p.ring_rows + 1));
+  };
+  const T *q = reinterpret_cast<const T *>(p.q) + b * p.q_bs + h * p.q_hs;
+  const T *K = reinterpret_cast<const T *>(p.k) + b * p.k_bs + h / p.group * p.k_hs, *V = reinterpret_cast<const T *>(p.v) + b * p.v_bs + h / p.group * p.v_hs;
+  int pos[kTiledRows], lo[kTiledRows];
+  float m[kTiledRows], l[kTiledRows], o[kTiledRows][kTiledWidth / 32];
+#pragma unroll
+  for (int r = 0; r < kTiledRows; ++r) {
+    const int i = i0 + warp * kTiledRows + r;
+    pos[r] = i < p.q_len ? base + i : -1;                // a row beyond the prompt sees nothing
+    lo[r] = lowest(base + i);
+    for (int d = lane; d < p.dk; d += 32) sq[r * p.dk + d] = i < p.q_len ? to_f32<T>(q[(long long)i * p.q_rs + d]) : 0.f;
+    m[r] = p.sinks ? p.sinks[h] * kLog2eLat : p.sink ? 0.f : -1e30f;
+    l[r] = p.sinks || p.sink ? 1.f : 0.f;
+#pragma unroll
+    for (int c = 0; c < kTiledWidth / 32; ++c) o[r][c] = 0.f;
+  }
+  const float r1 = p.r1 ? p.r1[h] : 0.f, r2 = p.r1 ? p.r2[h] : 0.f, slope = p.slopes ? p.slopes[h] * kLog2eLat : 0.f;
+  // positions that some row of the CTA sees: from the first row's lowest to the last row, and the kept ones
+  const int lo_cta = lowest(base + i0), hi_cta = base + min(i0 + kTiledWarps * kTiledRows, p.q_len) - 1;
+  const int from = p.keep > 0 ? min(first, lo_cta) : lo_cta;
+  for (int j0 = from; j0 <= hi_cta; j0 += kTiledKeys) {
+    if (j0 + kTiledKeys <= lo_cta && j0 >= first + p.keep) continue;
+    const int n = min(kTiledKeys, hi_cta + 1 - j0);
+    __syncthreads();
+    for (int jj = warp; jj < kTiledKeys; jj += kTiledWarps) {
+      const long long row = jj < n ? (j0 + jj) % p.ring_rows : 0;
+      for (int d = lane; d < p.dk; d += 32) sk[jj * kp + d] = jj < n ? to_f32<T>(K[row * p.k_rs + d]) : 0.f;
+      for (int d = lane; d < p.dv; d += 32) sv[jj * p.dv + d] = jj < n ? to_f32<T>(V[row * p.v_rs + d]) : 0.f;
+    }
+    __syncthreads();
+    float s[kTiledRows] = {};
+    const float4 *kr = reinterpret_cast<const float4 *>(sk + lane * kp);
+    for (int d = 0; d < p.dk / 4; ++d) {
+      const float4 kv = kr[d];
+#pragma unroll
+      for (int r = 0; r < kTiledRows; ++r) {
+        const float4 qv = reinterpret_cast<const float4 *>(sq + r * p.dk)[d];
+        s[r] = fmaf(qv.x, kv.x, s[r]);
+        s[r] = fmaf(qv.y, kv.y, s[r]);
+        s[r] = fmaf(qv.z, kv.z, s[r]);
+        s[r] = fmaf(qv.w, kv.w, s[r]);
+      }
+    }
+    const int j = j0 + lane;
+    float w[kTiledRows];
+    uint32_t mask[kTiledRows];
+#pragma unroll
+    for (int r = 0; r < kTiledRows; ++r) {
+      float x = s[r] * p.scale_log2;
+      if (p.inv_cap > 0.f) x = p.cap_log2 * capped_tanh<T>(s[r] * p.inv_cap);
+      if (p.r1) x -= r1 * log2f(fmaf(r2, (float)max(pos[r] - j, 0), 1.f));
+      x -= slope * (float)(pos[r] - j);
+      const bool seen = j >= first && j <= pos[r] && (j >= lo[r] || j < first + p.keep);
+      mask[r] = __ballot_sync(0xffffffffu, seen);
+      x = seen ? x : -INFINITY;
+      const float mn = fmaxf(m[r], warp_max(x)), alpha = exp2f(m[r] - mn);
+      w[r] = exp2f(x - mn);
+      m[r] = mn;
+      l[r] = l[r] * alpha + warp_sum(w[r]);
+#pragma unroll
+      for (int c = 0; c < kTiledWidth / 32; ++c) o[r][c] *= alpha;
+    }
+    reinterpret_cast<float4 *>(sp)[lane] = make_float4(w[0], w[1], w[2], w[3]);
+    __syncwarp();
+    for (int jj = 0; jj < n; ++jj) {
+      const float4 wv = reinterpret_cast<const float4 *>(sp)[jj];
+      const float wr[kTiledRows] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+      for (int c = 0; c < kTiledWidth / 32; ++c) {
+        if (c * 32 >= p.dv) break;
+        const float v = c * 32 + lane < p.dv ? sv[jj * p.dv + c * 32 + lane] : 0.f;
+#pragma unroll
+        for (int r = 0; r < kTiledRows; ++r)
+          if (mask[r] >> jj & 1u) o[r][c] = fmaf(wr[r], v, o[r][c]);      // (what a row does not see may hold anything)
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kTiledRows; ++r) {
+    const int i = i0 + warp * kTiledRows + r;
+    if (i >= p.q_len) continue;
+    const float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
+    T *out = reinterpret_cast<T *>(p.o) + b * p.o_bs + (long long)i * p.o_rs + h * p.o_hs;
+#pragma unroll
+    for (int c = 0; c < kTiledWidth / 32; ++c)
+      if (c * 32 + lane < p.dv) out[c * 32 + lane] = from_f32<T>(o[r][c] * inv);
+  }
+}
+
+template <typename T> int launch_tiled(const PlainParams &p, int B, cudaStream_t st) {
+  const size_t smem = tiled_smem(p.dk, p.dv);
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !configured[dev]) {
+    if (cudaFuncSetAttribute(attention_tiled_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled_smem(kTiledWidth, kTiledWidth)) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(EB_ECUDA, "attention_plain: cannot reserve shared memory");
+    }
+    configured[dev] = true;
+  }
+  constexpr int rows = kTiledWarps * kTiledRows;
+  launch_pdl(attention_tiled_kernel<T>, dim3((p.q_len + rows - 1) / rows, p.heads, B), dim3(kTiledWarps * 32), smem, st, p);
+  return check_launch("attention_plain");
+}
+
 template <typename T> int launch_plain(const PlainParams &p, int B, cudaStream_t st) {
+  // Few rows leave most of a tile's rows empty; a cache whose first positions lie in rows of their own is addressed per query.
+  if (p.q_len >= 8 && p.kept_rows == 0 && p.dk % 4 == 0 && p.dk <= kTiledWidth && p.dv <= kTiledWidth) return launch_tiled<T>(p, B, st);
   int warps = 4;
   const size_t per = (size_t)(p.dk + p.dv) * sizeof(float);
   while (warps > 1 && warps * per > 48 * 1024) warps >>= 1;

@@ -303,3 +303,35 @@ def test_gemm_f32_by_pieces(M, N, K):
     if M > 1 and N > 1:
         close(got2[M - 1, :N - 1] / 3e38, plain[M - 1, :N - 1] / 3e38, 1e-6)
     assert device_status()[0] == 0
+
+
+# From eight rows on 32 rows share tiles of 32 positions: rows around a tile, unequal head sizes, every rule of what is seen; what is not seen is NaN.
+@pytest.mark.parametrize("S,dk,dv", [(8, 4, 1), (33, 128, 128), (95, 96, 64), (200, 40, 33)])
+@pytest.mark.parametrize("rule", [dict(), dict(window=31), dict(chunk=16), dict(window=40, keep=5, cap=3.0)])
+def test_plain_attention_in_tiles(S, dk, dv, rule):
+    from energonai_b200.attention import attention_plain, attention_plain_capped, distance_slopes
+    B, H, G, scale = 2, 4, 2, 0.2
+    q, k, v = rnd(B, S, H * dk, dtype=F32), rnd(B, S, G * dk, seed=1, dtype=F32), rnd(B, S, G * dv, seed=2, dtype=F32)
+    first = [0, min(S - 1, 7)]
+    k[1, :first[1]] = v[1, :first[1]] = float("nan")
+    kw = dict(scale=scale, first=torch.tensor(first, dtype=torch.int32, device="cuda"), kv_heads=G)
+    kw.update(dict(sinks=torch.zeros(H, device="cuda")) if "chunk" in rule else dict(sink=True))
+    call = attention_plain_capped if "cap" in rule else attention_plain
+    if "cap" in rule:
+        kw["slopes"] = distance_slopes(H, "cuda")
+    got = call(q, k, v, H, dk, dv, **kw, **rule).double().cpu().view(B, S, H, dv)
+    i, j = torch.arange(S)[:, None], torch.arange(S)[None]
+    for b in range(B):
+        lo = torch.full((S, 1), first[b])
+        if rule.get("window"):
+            lo = torch.maximum(lo, i - rule["window"] + 1)
+        if rule.get("chunk"):
+            lo = torch.maximum(lo, lo + (i - lo).clamp(min=0) // rule["chunk"] * rule["chunk"])
+        seen = (j <= i) & (j >= first[b]) & ((j >= lo) | (j < first[b] + rule.get("keep", 0)))
+        for h in range(H):
+            kk, vv = (t[b, :, h // (H // G) * d:(h // (H // G) + 1) * d].double().cpu().nan_to_num() for t, d in ((k, dk), (v, dv)))
+            s = q[b, :, h * dk:(h + 1) * dk].double().cpu() @ kk.T * scale
+            if "cap" in rule:
+                s = rule["cap"] * torch.tanh(s / rule["cap"]) - kw["slopes"][h].double().cpu() * (i - j)
+            e = torch.where(seen, s.exp(), 0.0)
+            close(got[b, first[b]:, h], ((e @ vv) / (1 + e.sum(1, keepdim=True)))[first[b]:], 2e-6)
