@@ -7,8 +7,10 @@
 // framework kernels is nine launches of a few microseconds each on the critical path of a step
 // that is itself a chain of short launches.
 //
-// One CTA per sequence.  The position scalars are read by every CTA before it reports in; the
-// last CTA to report in advances them (so the launches of the next step find them advanced) and
+// A cluster of eight CTAs per sequence: what a step waits for is a row of 200 KB on its way into one SM and, one thread at a time, the trips of
+// its loads (one CTA of 256 threads took 15 to 43 us for 1 to 16 rows of 50272).  Each CTA reads an eighth, leaves its maximum in every other's
+// shared memory, and copies an eighth of the embedding of the token they all arrive at.  The position scalars are read by every CTA before it
+// reports in; the last CTA to report in advances them (so the launches of the next step find them advanced) and
 // rearms the counter.
 #include <cfloat>
 
@@ -17,7 +19,7 @@
 namespace eb {
 namespace {
 
-constexpr int kStepThreads = 256;
+constexpr int kStepThreads = 256, kStepCtas = 8, kStepWarps = kStepThreads / 32;
 
 struct StepParams {
   const void *logits;          // [batch][ld_logits], T
@@ -45,15 +47,21 @@ struct StepParams {
   int *counter;                // zero between launches
 };
 
+__device__ __forceinline__ uint32_t peer_addr(const void *p, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+
 // L: type of the logits, T: type of the embedding tables and of the output row
 template <typename L, typename T>
-__global__ void __launch_bounds__(kStepThreads) greedy_step_kernel(const StepParams p) {
-  __shared__ float s_val[kStepThreads / 32];
-  __shared__ int s_idx[kStepThreads / 32];
-  __shared__ int s_token;
+__global__ void __cluster_dims__(kStepCtas, 1, 1) __launch_bounds__(kStepThreads) greedy_step_kernel(const StepParams p) {
+  __shared__ float s_val[kStepWarps], c_val[kStepCtas];
+  __shared__ int s_idx[kStepWarps], c_idx[kStepCtas];
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (waited for before another CTA's memory is written)
   griddep_wait();
   griddep_launch();
-  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b = blockIdx.x / kStepCtas, rank = blockIdx.x % kStepCtas, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pos = p.kv_state[0], col = p.kv_state[1];
   const L *row = reinterpret_cast<const L *>(p.logits) + (long long)b * p.ld_logits;
 
@@ -63,47 +71,61 @@ __global__ void __launch_bounds__(kStepThreads) greedy_step_kernel(const StepPar
   auto take = [&](float v, int i) {
     if (v > best || (v == best && i < best_i)) { best = v; best_i = i; }
   };
-  constexpr int VEC = 16 / sizeof(L);
-  if ( p.ld_logits % VEC == 0 && (reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
-    const int packs = p.vocab / VEC;
-    for (int v = tid; v < packs; v += kStepThreads) {
-      Vec16<L> pk;
-      pk.load(row + (long long)v * VEC);
-      float f[VEC];
-      pk.unpack(f);
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) take(f[e], v * VEC + e);
-    }
-    for (int i = packs * VEC + tid; i < p.vocab; i += kStepThreads) take(to_f32<L>(row[i]), i);
-  } else {
-    for (int i = tid; i < p.vocab; i += kStepThreads) take(to_f32<L>(row[i]), i);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-    take(ov, oi);
-  }
-  if (lane == 0) { s_val[warp] = best; s_idx[warp] = best_i; }
-  __syncthreads();
-  if (warp == 0) {
-    best = lane < kStepThreads / 32 ? s_val[lane] : -FLT_MAX;
-    best_i = lane < kStepThreads / 32 ? s_idx[lane] : 0x7fffffff;
+  auto take_warp = [&]() {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, best, o);
       const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
       take(ov, oi);
     }
-    if (lane == 0) {
-      const int token = best_i == 0x7fffffff ? 0 : best_i;      // a row of NaNs: token 0
-      s_token = token;
-      if (p.tok) p.tok[b] = token;
-      if (col >= 0 && col < p.out_cols) p.out_ids[(long long)b * p.ld_out + col] = token;
+  };
+  // the row from its first 16-byte boundary on in packs, an eighth of them per CTA; what is left at its ends falls to the first CTA
+  constexpr int VEC = 16 / sizeof(L), kAhead = 4;
+  const int head = min(p.vocab, (int)((16 - (reinterpret_cast<uintptr_t>(row) & 15u)) % 16 / sizeof(L))), packs = (p.vocab - head) / VEC;
+  const int per = (packs + kStepCtas - 1) / kStepCtas, end = min(packs, (rank + 1) * per);
+  for (int v0 = rank * per + tid; v0 < end; v0 += kAhead * kStepThreads) {
+    Vec16<L> pk[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (v0 + u * kStepThreads < end) pk[u].load(row + head + (long long)(v0 + u * kStepThreads) * VEC);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (v0 + u * kStepThreads >= end) break;
+      float f[VEC];
+      pk[u].unpack(f);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) take(f[e], head + (v0 + u * kStepThreads) * VEC + e);
     }
   }
+  if (rank == 0) {
+    const int tail = head + packs * VEC + tid;
+    if (tid < head) take(to_f32<L>(row[tid]), tid);
+    if (tail < p.vocab) take(to_f32<L>(row[tail]), tail);
+  }
+  take_warp();
+  if (lane == 0) { s_val[warp] = best; s_idx[warp] = best_i; }
   __syncthreads();
-  const int token = s_token;
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if (warp == 0) {
+    best = lane < kStepWarps ? s_val[lane] : -FLT_MAX;
+    best_i = lane < kStepWarps ? s_idx[lane] : 0x7fffffff;
+    take_warp();
+    if (lane < kStepCtas) {
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_addr(c_val + rank, lane)), "f"(best) : "memory");
+      asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(peer_addr(c_idx + rank, lane)), "r"(best_i) : "memory");
+    }
+    __syncwarp();
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  best = -FLT_MAX;
+  best_i = 0x7fffffff;
+#pragma unroll
+  for (int r = 0; r < kStepCtas; ++r) take(c_val[r], c_idx[r]);
+  const int token = best_i == 0x7fffffff ? 0 : best_i;          // a row of NaNs: token 0
+  if (rank == 0 && tid == 0) {
+    if (p.tok) p.tok[b] = token;
+    if (col >= 0 && col < p.out_cols) p.out_ids[(long long)b * p.ld_out + col] = token;
+  }
 
   // embedding of the new token at the next position
   if (p.word_emb) {
@@ -113,7 +135,7 @@ __global__ void __launch_bounds__(kStepThreads) greedy_step_kernel(const StepPar
     const T *w = reinterpret_cast<const T *>(p.word_emb) + (mine ? local : 0) * p.hidden;
     const T *q = reinterpret_cast<const T *>(p.pos_emb) + (long long)next * p.hidden;
     T *o = reinterpret_cast<T *>(p.hidden_out) + (long long)b * p.ld_hidden;
-    for (int d = tid; d < p.hidden; d += kStepThreads) {
+    for (int d = rank * kStepThreads + tid; d < p.hidden; d += kStepCtas * kStepThreads) {
       const float wv = mine ? to_f32<T>(w[d]) : 0.f, pv = p.add_pos ? to_f32<T>(q[d]) : 0.f;
       o[d] = from_f32<T>(wv + pv);
     }
@@ -125,7 +147,7 @@ __global__ void __launch_bounds__(kStepThreads) greedy_step_kernel(const StepPar
                                                      : p.pair_rows;
     const T *w = reinterpret_cast<const T *>(p.pair_emb) + (r < 0 ? 0 : r) * p.hidden;
     T *o = reinterpret_cast<T *>(p.pair_out) + (long long)b * p.ld_pair;
-    for (int d = tid; d < p.hidden; d += kStepThreads) o[d] = w[d];
+    for (int d = rank * kStepThreads + tid; d < p.hidden; d += kStepCtas * kStepThreads) o[d] = w[d];
   }
 
   // every CTA has read the position scalars: the last one advances them
@@ -149,9 +171,9 @@ using namespace eb;
 namespace {
 template <typename L>
 void launch_step(int emb_dtype, int batch, cudaStream_t st, const StepParams &p) {
-  if (emb_dtype == EB_F32) launch_pdl(greedy_step_kernel<L, float>, dim3(batch), dim3(kStepThreads), 0, st, p);
-  else if (emb_dtype == EB_F16) launch_pdl(greedy_step_kernel<L, __half>, dim3(batch), dim3(kStepThreads), 0, st, p);
-  else launch_pdl(greedy_step_kernel<L, __nv_bfloat16>, dim3(batch), dim3(kStepThreads), 0, st, p);
+  if (emb_dtype == EB_F32) launch_pdl(greedy_step_kernel<L, float>, dim3(batch * kStepCtas), dim3(kStepThreads), 0, st, p);
+  else if (emb_dtype == EB_F16) launch_pdl(greedy_step_kernel<L, __half>, dim3(batch * kStepCtas), dim3(kStepThreads), 0, st, p);
+  else launch_pdl(greedy_step_kernel<L, __nv_bfloat16>, dim3(batch * kStepCtas), dim3(kStepThreads), 0, st, p);
 }
 }  // namespace
 

@@ -304,3 +304,22 @@ def test_greedy_step_tail(B, V, h, split, dtype):
     before = out_ids.clone()
     greedy_step(logits, out_ids, tok, kv, counter)
     assert torch.equal(out_ids, before) and kv.tolist() == [pos + 1, cols + 1]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("V", [1, 5, 31, 33, 257, 8191, 50257])
+def test_greedy_step_argmax_anywhere(V, dtype):
+    """The maximum in every eighth of a row and at its ends, rows that begin off 16 bytes, rows without a number above the lowest."""
+    from energonai_b200.step import greedy_step
+    at = sorted({0, V - 1, V // 2} | {min(V - 1, V * k // 8 + d) for k in range(8) for d in (0, 1)})
+    wide = torch.randn(len(at) + 2, V + 3, device="cuda", generator=torch.Generator(device="cuda").manual_seed(V)).clamp(-3, 3).to(dtype)
+    logits = wide[:, 1:V + 1]
+    for r, i in enumerate(at):
+        logits[r, i:] = torch.where(torch.arange(i, V, device="cuda") % 7 == i % 7, 9.0, logits[r, i:].float()).to(dtype)      # ties behind it
+    logits[-2], logits[-1] = float("nan"), -float("inf")
+    B = logits.shape[0]
+    out_ids, tok = torch.full((B, 3), -1, dtype=torch.int64, device="cuda"), torch.empty(B, dtype=torch.int64, device="cuda")
+    kv, counter = torch.tensor([4, 1], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    greedy_step(logits, out_ids, tok, kv, counter)
+    assert tok.tolist() == at + [0, 0] and out_ids[:, 1].tolist() == tok.tolist()
+    assert kv.tolist() == [5, 2] and counter.item() == 0
