@@ -86,7 +86,7 @@ def ptr(t):
 
 def stream_ptr():
     import torch
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())      # (without a Stream object per launch)
 
 
 def require_cuda(*tensors):
