@@ -297,6 +297,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           if (++stage == stages) { stage = 0; phase ^= 1u; }
         }
       }
+      // The hand-backs of the last stages, which no copy waits for: nothing orders them before the accumulator's signal, and the leader
+      // must not send them to a CTA that has left.  (A stage that was never filled counts as handed back.)
+      for (int s = 0; ok && s < stages; ++s) {
+        ok = mbar_wait(empty_bar + 8 * stage, phase ^ 1u, abort_flag, 15);
+        if (++stage == stages) { stage = 0; phase ^= 1u; }
+      }
     }
     __syncwarp();
   } else if (warp == 1) {

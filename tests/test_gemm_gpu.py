@@ -264,3 +264,21 @@ def test_gemm_pair_tiles(M, N, K, dtype):
     check_close(out, (plain + b.float())[:, :N - 24], dtype)
     check_close(tail, (plain + b.float())[:, N - 24:], torch.float32)
     status_ok()
+
+
+@pytest.mark.parametrize("M,N", [(1000, 4096), (3000, 6144)])
+def test_gemm_pair_tiles_one_behind_the_other(M, N):
+    """Launches that follow each other at once, with fewer k-blocks than the stages hold up to several rounds of them: whatever a stage's
+    hand-back finds when a CTA has left, the next kernel's barriers would show."""
+    from energonai_b200.gemm import gemm
+    w, x = torch.randn(N, 840, device="cuda").half(), torch.randn(M, 840, device="cuda").half()
+    for K in range(64, 841, 64):
+        a, b = x[:, :K], w[:, :K]
+        want = gemm(a, b, static_weight=True)
+        check_close(want, reference(a, b), torch.float16)
+        outs = [torch.empty_like(want) for _ in range(8)]
+        for _ in range(4):
+            for o in outs:
+                gemm(a, b, out=o, static_weight=True)
+        assert all(torch.equal(o, want) for o in outs)
+        status_ok()
