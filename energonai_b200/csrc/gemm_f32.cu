@@ -163,6 +163,11 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
       if (lane == 0) bar_arrive(full + 8 * stage);
       if (++stage == kF32Stages) { stage = 0; phase ^= 1u; }
     }
+    // the hand-backs of the last stages, which nothing orders before the sums' signal, do not find the CTA gone
+    for (int s = 0; s < kF32Stages; ++s) {
+      if (!__all_sync(0xffffffffu, bar_wait(empty + 8 * stage, phase ^ 1u, abort_flag, 5))) break;
+      if (++stage == kF32Stages) { stage = 0; phase ^= 1u; }
+    }
     for (int q = 0; q < kPasses; ++q)
       if (bad >> q & 1u) odd[q * 32 + row_in] = 1;
   } else {
