@@ -5,6 +5,8 @@
 // A single product may add a bias and apply xIELU to its first columns.  Two kernels:
 //   gemm_f32_tc_kernel   tensor cores, every operand split into three bf16 pieces
 //   gemm_f32_kernel      what it does not take: operands that 16-byte loads cannot read, a K below 64
+#include <cfloat>
+
 #include "common.cuh"
 #include "tc_ops.cuh"
 #include "xielu.cuh"
@@ -33,30 +35,73 @@ struct F32Params {
 // chain of fp32 multiply-adds: K = 64 7.7e-8 against 1.4e-7, K = 2048 1.3e-7 against 8.1e-7, K = 5632 1.9e-7 against 1.3e-6 (2-norm, normal operands).
 // Bound by the trip to L2 for a chunk's operands, of which one chunk is requested ahead (48 registers a thread), and by splitting them.
 // Warps 0-3 add up and store, 4-11 load, split and write the swizzled operand tiles, 12 issues the products.
-// An infinity, a NaN or a number that bf16 rounds to infinity has no such split: the outputs of its row are computed again by
-// multiply-adds.
+// An infinity, a NaN or a number that bf16 rounds to infinity has no such split, and where a product overflows, products of pieces
+// overflow each by itself, to either side: either way the sum is not finite.  Such outputs are computed again from the operands, by the
+// whole CTA, in 64 bits (all 128 x 64 of a tile with a K of 2048: 0.8 ms, at the rate of 64-bit multiply-adds; a row alone 20 us).
 constexpr int kF32Cols = 64, kF32Chunk = 64, kSplitWarps = 8, kF32TcThreads = 32 * (4 + kSplitWarps + 1), kF32Stages = 3;
 constexpr uint32_t kPlaneA = kRows * 128, kPlaneW = kF32Cols * 128, kF32StageBytes = 3 * (kPlaneA + kPlaneW);
 constexpr size_t kF32TcSmem = 1024 + 1024 + (size_t)kF32Stages * kF32StageBytes;
 
-// Pieces of two numbers, packed: hi, mid, lo.  Returns the magnitude bits of lo, at least 0x7f80 in a half whose number has no split.
+// Pieces of two numbers, packed.
 __device__ __forceinline__ uint32_t round2(float x0, float x1) {
   uint32_t v;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(x1), "f"(x0));
   return v;
 }
-__device__ __forceinline__ uint32_t split2(float x0, float x1, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
   hi = round2(x0, x1);
   x0 -= __uint_as_float(hi << 16); x1 -= __uint_as_float(hi & 0xffff0000u);
   mid = round2(x0, x1);
   lo = round2(x0 - __uint_as_float(mid << 16), x1 - __uint_as_float(mid & 0xffff0000u));
-  return lo & 0x7fff7fffu;
 }
 
 __device__ __forceinline__ void store_f32(const F32Params &p, float *C, int m, int n, float v, float up, float down) {
   v += p.bias ? p.bias[n] : 0.f;
   if (p.act_params && n < p.act_cols) v = xielu_exact(v, up, down);
   C[(long long)m * p.ldc + n] = v;
+}
+
+// The outputs of a tile that `redo` marks (a word of column bits per row), by all warps: one has 4 rows x 4 columns at a time, its lanes
+// share K.  A marked output costs its block's 8 rows of operands on their way from L2.
+__device__ __noinline__ void redo_marked(const F32Params &p, const float *A, const float *W, float *C, int m0, int n0, const unsigned long long *redo, float up,
+                                         float down) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int block = warp; block < kRows / 4 * (kF32Cols / 4); block += kF32TcThreads / 32) {
+    const int row = block / (kF32Cols / 4) * 4, col = block % (kF32Cols / 4) * 4;
+    uint32_t marked = 0;                                 // bit 4 r + c
+#pragma unroll
+    for (int r = 0; r < 4; ++r) marked |= ((uint32_t)(redo[row + r] >> col) & 15u) << (4 * r);
+    if (!marked) continue;
+    const float *a[4], *w[4];
+    double sum[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {                        // (rows and columns that are not there: the last ones, never marked)
+      a[i] = A + (long long)min(m0 + row + i, p.M - 1) * p.lda;
+      w[i] = W + (long long)min(n0 + col + i, p.N - 1) * p.ldw;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) sum[i][c] = 0.;
+    }
+    for (int k = lane * 4; k < p.K; k += 128) {
+      float4 x[4], y[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[i] = __ldg(reinterpret_cast<const float4 *>(a[i] + k));
+        y[i] = __ldg(reinterpret_cast<const float4 *>(w[i] + k));
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          sum[r][c] = fma((double)x[r].w, (double)y[c].w, fma((double)x[r].z, (double)y[c].z, fma((double)x[r].y, (double)y[c].y, fma((double)x[r].x, (double)y[c].x, sum[r][c]))));
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      double v = sum[i >> 2][i & 3];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == i && (marked >> i & 1u)) store_f32(p, C, m0 + row + (i >> 2), n0 + col + (i & 3), (float)v, up, down);
+    }
+  }
 }
 
 __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32Params p) {
@@ -67,7 +112,6 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
   const uint32_t full = s32(bars), empty = full + 8 * kF32Stages, tfull = empty + 8 * kF32Stages, tempty = tfull + 16;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kF32Stages + 4);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  volatile uint8_t *odd = smem + 512;                  // per row of A, then of W: holds a number that cannot be split
   const uint32_t tiles = s32(smem) + 1024;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * kRows, n0 = blockIdx.x * kF32Cols, chunks = (p.K + kF32Chunk - 1) / kF32Chunk;
@@ -78,7 +122,6 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (threadIdx.x < kRows + kF32Cols) odd[threadIdx.x] = 0;
   if (warp == 12) {
     __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)), "r"(2u * kF32Cols) : "memory");
@@ -99,6 +142,7 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
   const float *A = p.A + (p.tile_group ? 0 : group * p.a_gs), *W = p.W + group * p.w_gs;
   float *C = p.C + (p.tile_group ? 0 : group * p.c_gs);
   float acc[kF32Cols];
+  bool odd = false;
 
   if (!live) {
   } else if (warp < 4) {
@@ -138,7 +182,7 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
 #pragma unroll
     for (int q = 0; q < kPasses; ++q) load(q, 0);
     int stage = 0;
-    uint32_t phase = 0, bad = 0;
+    uint32_t phase = 0;
     for (int c = 0; c < chunks; ++c) {
       if (!__all_sync(0xffffffffu, bar_wait(empty + 8 * stage, phase ^ 1u, abort_flag, 2))) break;
       uint8_t *at = smem + 1024 + (size_t)stage * kF32StageBytes;
@@ -149,10 +193,10 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
         uint8_t *dst = at + (of_a ? 0 : 3 * kPlaneA) + row * 128 + ((unit ^ (row & 7)) << 4);
         const uint32_t plane = of_a ? kPlaneA : kPlaneW;
         uint4 hi, mid, lo;
-        uint32_t worst = __vmaxu2(split2(x[q][0].x, x[q][0].y, hi.x, mid.x, lo.x), split2(x[q][0].z, x[q][0].w, hi.y, mid.y, lo.y));
-        worst = __vmaxu2(worst, split2(x[q][1].x, x[q][1].y, hi.z, mid.z, lo.z));
-        worst = __vmaxu2(worst, split2(x[q][1].z, x[q][1].w, hi.w, mid.w, lo.w));
-        bad |= (worst + 0x00800080u) & 0x80008000u ? 1u << q : 0u;             // (a half of 0x7f80 or more)
+        split2(x[q][0].x, x[q][0].y, hi.x, mid.x, lo.x);
+        split2(x[q][0].z, x[q][0].w, hi.y, mid.y, lo.y);
+        split2(x[q][1].x, x[q][1].y, hi.z, mid.z, lo.z);
+        split2(x[q][1].z, x[q][1].w, hi.w, mid.w, lo.w);
         *reinterpret_cast<uint4 *>(dst) = hi;
         *reinterpret_cast<uint4 *>(dst + plane) = mid;
         *reinterpret_cast<uint4 *>(dst + 2 * plane) = lo;
@@ -168,8 +212,6 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
       if (!__all_sync(0xffffffffu, bar_wait(empty + 8 * stage, phase ^ 1u, abort_flag, 5))) break;
       if (++stage == kF32Stages) { stage = 0; phase ^= 1u; }
     }
-    for (int q = 0; q < kPasses; ++q)
-      if (bad >> q & 1u) odd[q * 32 + row_in] = 1;
   } else {
     // ---------------- products ----------------
     constexpr uint32_t idesc = tc_idesc(kF32Cols, 1);
@@ -202,29 +244,34 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * kF32Cols) : "memory");
   }
-  if (!live || warp >= 4 || *abort_flag) return;
-  const int m = m0 + warp * 32 + lane;
-  if (m >= p.M) return;
-#pragma unroll
-  for (int j = 0; j < kF32Cols; ++j) {
-    if (!(odd[warp * 32 + lane] | odd[kRows + j]) || n0 + j >= p.N) continue;
-    float v = 0.f;
-    for (int k = 0; k < p.K; ++k) v = fmaf(A[(long long)m * p.lda + k], W[(long long)(n0 + j) * p.ldw + k], v);
-    acc[j] = v;
-  }
+  if (!live || *abort_flag) return;                    // (uniform)
   float up = 0.f, down = 0.f;
   if (p.act_params) { up = p.act_params[0]; down = p.act_params[1]; }
-  const bool wide = !p.bias && !p.act_params && ((uintptr_t)C & 15) == 0 && p.ldc % 4 == 0;
+  unsigned long long *redo = reinterpret_cast<unsigned long long *>(smem + 1024);      // per row: the columns to compute again (the stages are free)
+  if (warp < 4) {
+    const int row = warp * 32 + lane, m = m0 + row;
+    unsigned long long again = 0;
+    if (m < p.M) {
 #pragma unroll
-  for (int j = 0; j < kF32Cols; j += 4) {
-    if (wide && n0 + j + 4 <= p.N) {
-      *reinterpret_cast<float4 *>(C + (long long)m * p.ldc + n0 + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-    } else {
+      for (int j = 0; j < kF32Cols; ++j)
+        if (n0 + j < p.N && !(fabsf(acc[j]) <= FLT_MAX)) again |= 1ull << j;
+      const bool wide = !p.bias && !p.act_params && ((uintptr_t)C & 15) == 0 && p.ldc % 4 == 0;
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (n0 + j + e < p.N) store_f32(p, C, m, n0 + j + e, acc[j + e], up, down);
+      for (int j = 0; j < kF32Cols; j += 4) {
+        if (wide && n0 + j + 4 <= p.N) {
+          *reinterpret_cast<float4 *>(C + (long long)m * p.ldc + n0 + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (n0 + j + e < p.N) store_f32(p, C, m, n0 + j + e, acc[j + e], up, down);
+        }
+      }
     }
+    redo[row] = again;
+    odd = again != 0;
   }
+  if (!__syncthreads_or(odd)) return;
+  redo_marked(p, A, W, C, m0, n0, redo, up, down);
 }
 
 // ---- any operands: a tiled CUDA-core kernel, 64 x 64 outputs per CTA ----------------------------------------------------------------

@@ -335,3 +335,26 @@ def test_plain_attention_in_tiles(S, dk, dv, rule):
                 s = rule["cap"] * torch.tanh(s / rule["cap"]) - kw["slopes"][h].double().cpu() * (i - j)
             e = torch.where(seen, s.exp(), 0.0)
             close(got[b, first[b]:, h], ((e @ vv) / (1 + e.sum(1, keepdim=True)))[first[b]:], 2e-6)
+
+
+def test_gemm_f32_products_that_overflow():
+    """A sum that leaves the range is an infinity of the right sign however its operands split; one that ends inside it is a number (the
+    bound: a product of two fp32 numbers rounded once).  Whole rows without a split, next to rows that have one."""
+    from energonai_b200.gemm import device_status, gemm_f32
+    a, w = rnd(70, 512, dtype=F32), rnd(96, 512, seed=1, dtype=F32)
+    want = ((5e24 * a).double() @ (5e24 * w).double().T).float()
+    assert want.isinf().any() and torch.equal(gemm_f32(5e24 * a, 5e24 * w), want)
+    a1, w1 = torch.zeros(70, 64, device="cuda"), torch.zeros(96, 64, device="cuda")
+    a1[:, 3], w1[:, 3] = 2.0 ** 64 * torch.linspace(0.98, 0.9999, 70, device="cuda"), 2.0 ** 63.9999
+    want = (a1.double() @ w1.double().T).float()
+    got = gemm_f32(a1, w1)
+    assert torch.equal(got.isfinite(), want.isfinite()) and float((got - want).abs().max()) <= 2.0 ** -23 * float(want.abs().max())
+    good = gemm_f32(a, w)
+    a[::2] = float("nan")
+    a[1], a[3, 5] = -3.4e38, float("inf")
+    got, want = gemm_f32(a, w), (a.double() @ w.double().T).float()
+    assert got[::2].isnan().all() and torch.equal(got[5::2], good[5::2]) and torch.equal(got[3], want[3])
+    finite = want[1].isfinite()
+    assert torch.equal(got[1][~finite], want[1][~finite])
+    close(got[1][finite] / 3e38, want[1][finite] / 3e38, 1e-6)
+    assert device_status()[0] == 0
