@@ -20,9 +20,10 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
               "--use_fast_math", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",
               "-diag-suppress", "177,550"]
 # Recurrences add up the logarithms of their gates over a whole sequence: an approximation's bias would
-# add up with them, so these files get the accurate functions; so do angles that grow with the position.
+# add up with them, so these files get the accurate functions; so do angles that grow with the position, and the
+# 32-bit products, whose operands' remainders may lie below the normal range.
 ACCURATE = {"matrix_memory.cu", "matrix_memory_tc.cu", "decay_memory.cu", "decay_memory_tc.cu", "attention_rotary.cu", "latent_inputs.cu",
-            "selective_scan.cu"}
+            "selective_scan.cu", "gemm_f32.cu"}
 
 
 def nvcc_flags(source):

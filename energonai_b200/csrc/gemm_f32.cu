@@ -35,9 +35,14 @@ struct F32Params {
 // chain of fp32 multiply-adds: K = 64 7.7e-8 against 1.4e-7, K = 2048 1.3e-7 against 8.1e-7, K = 5632 1.9e-7 against 1.3e-6 (2-norm, normal operands).
 // Bound by the trip to L2 for a chunk's operands, of which one chunk is requested ahead (48 registers a thread), and by splitting them.
 // Warps 0-3 add up and store, 4-11 load, split and write the swizzled operand tiles, 12 issues the products.
-// An infinity, a NaN or a number that bf16 rounds to infinity has no such split, and where a product overflows, products of pieces
-// overflow each by itself, to either side: either way the sum is not finite.  Such outputs are computed again from the operands, by the
-// whole CTA, in 64 bits (all 128 x 64 of a tile with a K of 2048: 0.8 ms, at the rate of 64-bit multiply-adds; a row alone 20 us).
+// Some outputs are computed again from the operands, by the whole CTA, in 64 bits (all 128 x 64 of a tile with a K of 2048: 0.8 ms, at
+// the rate of 64-bit multiply-adds):
+//   not finite   an infinity or a number that bf16 rounds to infinity has no such split, and where a product overflows, products of
+//                pieces overflow each by itself, to either side
+//   small        below 2^-100 a number's lower pieces, or what they are multiplied to, can lie below the normal range (2^-126; bf16 ends at
+//                2^-133): an absolute error of up to 2^-126 per term and unit of the other operand.  That counts where one side's row is that
+//                small throughout, or the sum is not 2^24 times what the errors can add up to.
+// A NaN among the operands stays one in the pieces and in the sum, which is then right as it is.
 constexpr int kF32Cols = 64, kF32Chunk = 64, kSplitWarps = 8, kF32TcThreads = 32 * (4 + kSplitWarps + 1), kF32Stages = 3;
 constexpr uint32_t kPlaneA = kRows * 128, kPlaneW = kF32Cols * 128, kF32StageBytes = 3 * (kPlaneA + kPlaneW);
 constexpr size_t kF32TcSmem = 1024 + 1024 + (size_t)kF32Stages * kF32StageBytes;
@@ -53,6 +58,13 @@ __device__ __forceinline__ void split2(float x0, float x1, uint32_t &hi, uint32_
   x0 -= __uint_as_float(hi << 16); x1 -= __uint_as_float(hi & 0xffff0000u);
   mid = round2(x0, x1);
   lo = round2(x0 - __uint_as_float(mid << 16), x1 - __uint_as_float(mid & 0xffff0000u));
+}
+
+// The largest magnitude; a NaN stays.
+__device__ __forceinline__ float largest(float x, float y, float z) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(y), "f"(z));
+  return r;
 }
 
 __device__ __forceinline__ void store_f32(const F32Params &p, float *C, int m, int n, float v, float up, float down) {
@@ -112,6 +124,7 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
   const uint32_t full = s32(bars), empty = full + 8 * kF32Stages, tfull = empty + 8 * kF32Stages, tempty = tfull + 16;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * kF32Stages + 4);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  float *top = reinterpret_cast<float *>(smem + 256);  // per row of A, then of W: its largest magnitude, or NaN
   const uint32_t tiles = s32(smem) + 1024;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * kRows, n0 = blockIdx.x * kF32Cols, chunks = (p.K + kF32Chunk - 1) / kF32Chunk;
@@ -169,6 +182,7 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
     constexpr int kPasses = (kRows + kF32Cols) / 32;
     const int t = threadIdx.x - 128, unit = t & 7, row_in = t >> 3;
     float4 x[kPasses][2];
+    float most[kPasses] = {};
     auto load = [&](int q, int c) {
       const int row = q * 32 + row_in, k = c * kF32Chunk + unit * 8;
       const bool of_a = q < kRows / 32;
@@ -197,6 +211,7 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
         split2(x[q][0].z, x[q][0].w, hi.y, mid.y, lo.y);
         split2(x[q][1].x, x[q][1].y, hi.z, mid.z, lo.z);
         split2(x[q][1].z, x[q][1].w, hi.w, mid.w, lo.w);
+        most[q] = largest(largest(x[q][0].x, x[q][0].y, x[q][0].z), largest(x[q][0].w, x[q][1].x, x[q][1].y), largest(x[q][1].z, x[q][1].w, most[q]));
         *reinterpret_cast<uint4 *>(dst) = hi;
         *reinterpret_cast<uint4 *>(dst + plane) = mid;
         *reinterpret_cast<uint4 *>(dst + 2 * plane) = lo;
@@ -211,6 +226,12 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
     for (int s = 0; s < kF32Stages; ++s) {
       if (!__all_sync(0xffffffffu, bar_wait(empty + 8 * stage, phase ^ 1u, abort_flag, 5))) break;
       if (++stage == kF32Stages) { stage = 0; phase ^= 1u; }
+    }
+#pragma unroll
+    for (int q = 0; q < kPasses; ++q) {
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) most[q] = largest(most[q], __shfl_xor_sync(0xffffffffu, most[q], o), 0.f);
+      if (unit == 0) top[q * 32 + row_in] = most[q];
     }
   } else {
     // ---------------- products ----------------
@@ -251,10 +272,25 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
   if (warp < 4) {
     const int row = warp * 32 + lane, m = m0 + row;
     unsigned long long again = 0;
+    const uint32_t w0 = __float_as_uint(top[kRows + lane]), w1 = __float_as_uint(top[kRows + 32 + lane]);      // (their order is that of the numbers; a NaN above all)
+    const float tw_least = __uint_as_float(__reduce_min_sync(0xffffffffu, min(w0, w1))), tw_most = __uint_as_float(__reduce_max_sync(0xffffffffu, max(w0, w1)));
     if (m < p.M) {
+      // Mostly the whole row is fine by its least and largest sum.
+      const float ta = top[row], least = (float)p.K * 0x1p-102f;
+      float v_least = FLT_MAX, v_most = 0.f;
 #pragma unroll
-      for (int j = 0; j < kF32Cols; ++j)
-        if (n0 + j < p.N && !(fabsf(acc[j]) <= FLT_MAX)) again |= 1ull << j;
+      for (int j = 0; j < kF32Cols; ++j) {
+        v_least = fminf(v_least, fabsf(acc[j]));
+        v_most = largest(v_most, acc[j], 0.f);
+      }
+      if (!(v_most <= FLT_MAX && (ta == 0.f || (fminf(ta, tw_least) >= 0x1p-100f && v_least >= fmaxf(0x1p-100f, least * fmaxf(ta, tw_most)))))) {
+#pragma unroll
+        for (int j = 0; j < kF32Cols; ++j) {
+          const float tw = top[kRows + j], v = fabsf(acc[j]), small = fminf(ta, tw);
+          const bool lost = small > 0.f && (small < 0x1p-100f || (v < fmaxf(0x1p-100f, least * fmaxf(ta, tw)) && (v > 0.f || ta * tw < 0x1p-100f)));
+          if (n0 + j < p.N && !isnan(ta) && !isnan(tw) && (!(v <= FLT_MAX) || lost)) again |= 1ull << j;
+        }
+      }
       const bool wide = !p.bias && !p.act_params && ((uintptr_t)C & 15) == 0 && p.ldc % 4 == 0;
 #pragma unroll
       for (int j = 0; j < kF32Cols; j += 4) {

@@ -358,3 +358,33 @@ def test_gemm_f32_products_that_overflow():
     assert torch.equal(got[1][~finite], want[1][~finite])
     close(got[1][finite] / 3e38, want[1][finite] / 3e38, 1e-6)
     assert device_status()[0] == 0
+
+
+@pytest.mark.parametrize("K", [64, 2052])
+def test_gemm_f32_small_operands(K):
+    """Rows down to the end of the normal range on either side, all together and one by one, beside rows of ordinary size: 1e-6 of the 64-bit
+    result, per row and column (the product of the smallest falls below the normal range: half its last place, 2^-150, per output beside it)."""
+    from energonai_b200.gemm import device_status, gemm_f32
+    a, w = rnd(70, K, dtype=F32), rnd(96, K, seed=1, dtype=F32)
+    want = a.double() @ w.double().T
+    rel = lambda y, ref, dim: ((y.double() - ref).norm(dim=dim) / ref.norm(dim=dim)).max()
+    for e in (-28, -30, -32, -33, -34, -35, -36):
+        x, v = a * 10.0 ** e, w * 10.0 ** e
+        for y, ref in ((gemm_f32(x, w), x.double() @ w.double().T), (gemm_f32(a, v), a.double() @ v.double().T)):
+            assert rel(y, ref, 0) < 1e-6 and rel(y, ref, 1) < 1e-6
+        s = torch.where(torch.arange(70, device="cuda") % 3 == 1, 10.0 ** e, 1.0)[:, None]
+        assert rel(gemm_f32(a * s, w), (a * s).double() @ w.double().T, 1) < 1e-6
+        half = 10.0 ** (e / 2)                                        # operands of ordinary size, a product that is not
+        assert rel(gemm_f32(a * half, w * half), (a * half).double() @ (w * half).double().T, 1) < 1e-6
+    x = a * 1e-37
+    assert float((gemm_f32(x, w).double() - x.double() @ w.double().T).abs().max()) < 1e-6 * float((x.double() @ w.double().T).abs().max()) + 2.0 ** -149
+    # small and ordinary numbers in one row, the ordinary ones against zeros
+    x, v = a * 1e-35, w.clone()
+    x[:, 7], v[:, 7] = 1.0, 0.0
+    assert rel(gemm_f32(x, v), x.double() @ v.double().T, 1) < 1e-6
+    # zeros stay zeros, rows of them and single sums
+    x, v = a.clone(), torch.zeros_like(w)
+    x[5], v[3, 2] = 0.0, 1.0
+    got = gemm_f32(x, v)
+    assert torch.equal(got[:, 3], x[:, 2]) and not got[:, :3].any() and not got[:, 4:].any()
+    assert rel(gemm_f32(a, w), want, 1) < 1e-6 and device_status()[0] == 0
