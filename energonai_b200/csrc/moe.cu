@@ -335,6 +335,12 @@ extern "C" int eb_moe_permute(const void *x, long long ldx, int n2, int dtype, i
   EB_REQUIRE(n2 > 0 && n2 % per == 0 && ldx % per == 0 && ldo % per == 0 && ldx >= n2 && ldo >= n2, "moe_permute: rows must be whole 16-byte packs");
   EB_REQUIRE(aligned16(x) && aligned16(out), "moe_permute: pointers must be 16-byte aligned");
   EB_REQUIRE(tokens > 0 && top > 0 && max_rows > 0, "moe_permute: bad sizes");
+  // 32-bit products look at what their rows hold: whatever lay in the rows that fill up a tile would decide their time.  (Zeros stay
+  // zeros through the units.)
+  if (dtype == EB_F32 && cudaMemset2DAsync(out, (size_t)ldo * 4, 0, (size_t)n2 * 4, (size_t)max_rows, as_stream(stream)) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(EB_ECUDA, "moe_permute: cannot clear the rows");
+  }
   launch_pdl(moe_permute_kernel, dim3((tokens + 7) / 8), dim3(kPermuteThreads), 0, as_stream(stream), reinterpret_cast<const uint4 *>(x),
              ldx / per, n2 / per, tokens, top, idx, ranks, offsets, rows, reinterpret_cast<uint4 *>(out), ldo / per, max_rows);
   return check_launch("moe_permute");

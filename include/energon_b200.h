@@ -422,7 +422,8 @@ EB_API int eb_moe_route_rule(const float *logits, long long ld, int tokens, int 
 EB_API int eb_moe_plan(int32_t *counts, int experts, int32_t *offsets, int32_t *tile_group, int max_tiles, int32_t *live_tiles,
                 void *stream);
 
-/* rows[t][k] = offsets[idx] + rank (or -1: no index or no rank) and out[rows[t][k]] = x[t]. */
+/* rows[t][k] = offsets[idx] + rank (or -1: no index or no rank) and out[rows[t][k]] = x[t]; the other of the max_rows rows
+ * become zeros if x is fp32 and keep what they hold otherwise. */
 EB_API int eb_moe_permute(const void *x, long long ldx, int n2, int dtype, int tokens, int top, const int32_t *idx,
                    const int32_t *ranks, const int32_t *offsets, int32_t *rows, void *out, long long ldo, int max_rows,
                    void *stream);

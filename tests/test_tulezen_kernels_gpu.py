@@ -388,3 +388,37 @@ def test_gemm_f32_small_operands(K):
     got = gemm_f32(x, v)
     assert torch.equal(got[:, 3], x[:, 2]) and not got[:, :3].any() and not got[:, 4:].any()
     assert rel(gemm_f32(a, w), want, 1) < 1e-6 and device_status()[0] == 0
+
+
+def test_mixture_in_32_bit_fills_its_tiles_with_zeros():
+    """The rows that fill up an expert's tiles take no part, but their product is formed: zeros in, zeros out, whatever the memory held (here
+    NaN), in a captured run too."""
+    from energonai_b200.moe import SortedRows, grouped_gemm, new_counts, route
+    T, W, E, top, ff = 37, 256, 12, 3, 64
+    x, router = rnd(T, W, dtype=F32), rnd(E, W, seed=1, dtype=F32)
+    up, down = rnd(E, 2 * ff, W, seed=2, scale=W ** -0.5, dtype=F32), rnd(E, W, ff, seed=3, scale=ff ** -0.5, dtype=F32)
+    counts = new_counts(E, "cuda")
+
+    def run():
+        idx, w, ranks = route(x @ router.T, E, top, counts=counts)
+        plan = SortedRows(x, idx, ranks, counts)
+        act = grouped_gemm(plan.x, up, plan, gate=(7.0, 1.702))
+        return idx, plan, act, grouped_gemm(act, down, plan)
+    held = [torch.full((1 << 22,), float("nan"), device="cuda") for _ in range(8)]
+    del held                                                          # (what the next allocations are cut from)
+    outs = [run()]
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        outs.append(run())
+    outs[1][1].x.fill_(float("nan"))
+    g.replay()
+    for idx, plan, act, y in outs:
+        live = int(plan.live_tiles) * 128
+        used = torch.zeros(live, dtype=torch.bool, device="cuda")
+        used[plan.rows.flatten().long()] = True
+        assert 0 < int(used.sum()) == T * top < live
+        for t in (plan.x, act, y):
+            assert not t[:live][~used].any()
+        assert torch.equal(plan.x[plan.rows.long()], x[:, None].expand(T, top, W))
+        got = y[plan.rows.long()]
+        assert got.isfinite().all() and torch.equal(got, outs[0][3][outs[0][1].rows.long()])
