@@ -4,7 +4,7 @@
 //   groups > 1           blockIdx.z = group: strides between the groups' operands
 // A single product may add a bias and apply xIELU to its first columns.  Two kernels:
 //   gemm_f32_tc_kernel   tensor cores, every operand split into three bf16 pieces
-//   gemm_f32_kernel      what it does not take: operands that 16-byte loads cannot read, a K below 64
+//   gemm_f32_kernel      what it does not take: operands that 16-byte loads cannot read, a K below 64 or, for many columns, 128
 #include <cfloat>
 
 #include "common.cuh"
@@ -384,9 +384,12 @@ extern "C" int eb_gemm_f32(const float *A, long long lda, long long a_group_stri
   p.bias = bias; p.act_cols = act_cols; p.act_params = act_params;
   cudaStream_t st = as_stream(stream);
   // 16-byte loads need rows that begin and end on 16 bytes, and below a chunk the multiply-adds are the closer ones (K = 4: 4.0e-8 against
-  // 4.6e-8).  However many rows there are: a row's result is the same in every batch.  333 x 11264 x 2048: 881 us by multiply-adds, 195 so; one
-  // row x 2048 x 2048 151 and 43.
-  const bool packs = K >= kF32Chunk && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && a_group_stride % 4 == 0 && w_group_stride % 4 == 0 && aligned16(A) && aligned16(W);
+  // 4.6e-8).  However many rows there are: a row's result is the same in every batch.  333 x 11264 x 2048: 881 us by multiply-adds, 202 so; one
+  // row x 2048 x 2048 149 and 39.  With a short K a tile is little but the way in and out, which tiles of one SM go one after the other, while several
+  // of the multiply-add kernel's share it: beyond a wave of columns the line lies at two chunks (one row x 32768: K = 64 17 us against 24, K = 96 24
+  // against 28, K = 128 30 against 28).
+  const bool many = (long long)((N + kF32Cols - 1) / kF32Cols) * groups > sm_count();
+  const bool packs = K >= (many ? 2 : 1) * kF32Chunk && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && a_group_stride % 4 == 0 && w_group_stride % 4 == 0 && aligned16(A) && aligned16(W);
   if (packs) {
     static bool configured[64] = {};
     int dev = 0;

@@ -422,3 +422,17 @@ def test_mixture_in_32_bit_fills_its_tiles_with_zeros():
         assert torch.equal(plan.x[plan.rows.long()], x[:, None].expand(T, top, W))
         got = y[plan.rows.long()]
         assert got.isfinite().all() and torch.equal(got, outs[0][3][outs[0][1].rows.long()])
+
+
+@pytest.mark.parametrize("N,heads", [(150 * 64, 1), (160, 50)])
+def test_gemm_f32_short_k_of_many_columns(N, heads):
+    """More column tiles than SMs: by multiply-adds below two chunks of K, bit for bit what rows that begin off 16 bytes get; by pieces from there on."""
+    from energonai_b200.moe import per_head
+    for M in (1, 130):
+        for K, pieces in ((64, False), (124, False), (128, True)):
+            a, w = rnd(M, heads * K, dtype=F32), rnd(heads, N, K, seed=1, scale=K ** -0.5, dtype=F32)
+            odd = torch.zeros(M, heads * K + 1, device="cuda")[:, 1:]
+            odd.copy_(a)
+            got, plain = per_head(a, w), per_head(odd, w)
+            assert torch.equal(got, plain) is not pieces and torch.equal(got[-1:], per_head(a[-1:], w))
+            close(got.view(M, heads, N), torch.einsum("mhk,hnk->mhn", a.view(M, heads, K).double(), w.double()), 1e-6)
