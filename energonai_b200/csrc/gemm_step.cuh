@@ -8,11 +8,14 @@
 // products are far below either's rate.  The weights of the first eight k-steps of every warp are requested
 // before the preceding kernel of the stream is waited for, so behind that wait a launch consists of one L2
 // trip for the activations (one cp.async per 16 bytes, all at once), the MMAs, one sum over the warps in shared memory
-// and the store.  At most 128 registers, so that the next launch's CTAs fit beside these and fetch their weights meanwhile.
+// and the store.  The sums of a slice's first 256 columns wait in shared memory for the others: mma.sync truncates as it accumulates, and with 512
+// columns in one accumulator a K of 4096 was off by 6.4e-7 where the tcgen05 form is by 3.5e-7 (fp16 operands, 2-norm; now 3.4e-7; a K of 768 1.6e-7
+// against 9.5e-7).  At most 128 registers, so that the next launch's CTAs fit beside these and fetch their weights meanwhile.
 // Launches one behind the other, each with other weights (tcgen05 form before): 768 x 768 with one row 5.2 -> 2.4 us, 2304 x 768
 // with eight rows and the LayerNorm 5.4 -> 3.3, 768 x 3072 7.7 -> 4.4, 2048 x 2048 with 16 rows 7.3 -> 5.1.
 constexpr int kStepWarps = 8, kStepThreads = kStepWarps * 32;
 constexpr int kStepUnroll = 4;                      // k-steps (32 columns of a warp's slice) per weight request
+constexpr int kStepRun = 256;                       // columns that a warp adds up in one accumulator
 constexpr int kStepPart = 33;                       // floats per accumulator element and warp (32 lanes and one against bank conflicts)
 
 struct StepGeometry {
@@ -141,9 +144,21 @@ gemm_step_kernel(const GemmParams p, const void *weights, long long ldw, int sli
   float acc[NT][4];
   float b_n = 0.f, colsum = 0.f;
   T r_mn[kPer];
-  auto begin_tile = [&]() {
+  // The lane's accumulators to its places in this tile's half of `part`, on top of what they hold or not.  (The half's last readers have passed the
+  // preceding tile's rendezvous, and so has this warp.)
+  auto leave_sums = [&](bool add) {
+    float *mine = part + (size_t)(buf * kStepWarps + warp) * (NT * 4) * kStepPart + lane;
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) mine[(j * 4 + e) * kStepPart] = add ? mine[(j * 4 + e) * kStepPart] + acc[j][e] : acc[j][e];
+  };
+  auto clear_sums = [&]() {
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+  };
+  auto begin_tile = [&]() {
+    clear_sums();
     const int n = tile * 16 + n_local;
     const bool n_ok = n < p.N && !p.gated;
     b_n = !n_ok ? 0.f : fold ? __ldg(p.ln_bias + n) : bias ? to_f32<T>(bias[n]) : 0.f;
@@ -155,11 +170,7 @@ gemm_step_kernel(const GemmParams p, const void *weights, long long ldw, int sli
     }
   };
   auto finish_tile = [&]() {
-    float *mine = part + (size_t)(buf * kStepWarps + warp) * (NT * 4) * kStepPart;
-#pragma unroll
-    for (int j = 0; j < NT; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) mine[(j * 4 + e) * kStepPart + lane] = acc[j][e];
+    leave_sums(slice > kStepRun);
     if (fold && first) {
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
@@ -253,6 +264,9 @@ gemm_step_kernel(const GemmParams p, const void *weights, long long ldw, int sli
       chunk = 0;
       tile += gridDim.x;
       if (tile < tiles) begin_tile();
+    } else if (chunk == kStepRun / (32 * U)) {            // (once: a slice has at most 512 columns)
+      leave_sums(false);
+      clear_sums();
     }
     return tile < tiles;
   };

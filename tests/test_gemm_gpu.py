@@ -282,3 +282,18 @@ def test_gemm_pair_tiles_one_behind_the_other(M, N):
                 gemm(a, b, out=o, static_weight=True)
         assert all(torch.equal(o, want) for o in outs)
         status_ok()
+
+
+# A warp's slice of K above 256 columns: one column more, part of a second run, a whole one; rows in ones, eights, sixteens and thirty-twos.
+@pytest.mark.parametrize("M,N,K", [(8, 520, 2056), (32, 520, 2304), (8, 1024, 3072), (2, 1024, 4096), (16, 1024, 4096)])
+def test_gemm_few_rows_long_k(M, N, K):
+    """No run of accumulations is longer than that of a K of 2048, so the sums are as close to 64 bits as those (3.5e-7, each
+    accumulation truncating; 512 columns in one run: 6.4e-7).  And a row's sum does not depend on how many rows take this form."""
+    from energonai_b200.gemm import gemm
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, w = torch.randn(M, K, device="cuda", generator=g).half(), (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).half()
+    got, want = gemm(x, w, out_dtype=torch.float32), x.double() @ w.double().t()
+    assert float((got - want).norm() / want.norm()) < 4e-7
+    for m in (1, M // 2 + 1):
+        assert torch.equal(gemm(x[-m:], w, out_dtype=torch.float32), got[-m:])
+    status_ok()
