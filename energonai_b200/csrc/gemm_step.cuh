@@ -28,15 +28,19 @@ struct StepGeometry {
 // 26.9), but in a model the tcgen05 form asks for more of its weights while the attention before it still runs.  33 steps of two layers of 12 h^2
 // weights, 8 rows: h = 1536 5.4 -> 5.2 ms, h = 3072 with all of them in this form 7.5 -> 8.6, with the square ones alone 7.7 -> 8.0; a head of 50257 x 768
 // with 8 rows, 18.5 us against 21.3, is better off in this form (31 steps of 12 layers 11.9 ms against 12.6).  A longer K
-// leaves a CTA too little in flight (2048 x 5632: 17.4 us against 11.7).  With more rows the reads of the activations from shared memory, once per
-// 16 weight rows, set the
+// leaves a CTA too little in flight (2048 x 5632: 17.4 us against 11.7), and with a short one a tile is little but its rendezvous and sums, of which a CTA
+// should not have many one after the other (8192 x 256 3.3 us against 3.8, 16384 x 256 5.4 against 4.8, 50264 x 512 13.9 against 13.3).
+// With more rows the reads of the activations from shared memory, once per 16 weight rows, set the
 // pace: 4096 x 2048 elements are the line for 16 rows (2048 x 2048: 5.1 against 7.3; 3072 x 3072: 10.9 against 8.1), 2048 x 2048
-// for 32 (7.3 against 10.2), and a CTA has to be done with one tile (16 rows, two CTAs per SM: 4096 x 1024 5.4 us against 6.5, 50264 x 768
-// 22.4 against 21.6; 32 rows, one CTA: 2304 x 768 6.4 against 6.8, 3072 x 1024 10.8 against 7.6).
+// for 32 (7.3 against 10.2), and a CTA has to be done with one tile.  Of 16 rows two CTAs run well side by side up to a K of 2048 (4096 x 1024 5.4 us
+// against 6.5, 3072 x 2048 6.9 against 9.1, 3072 x 2304 8.0 against 7.9, 2720 x 2816 11.4 against 9.3; from K = 2817 on one fills the shared memory), of 32 rows
+// one (2304 x 768 6.4 against 6.8, 3072 x 1024 10.8 against 7.6).
+// A row is summed in another order here than in the tcgen05 form, so its rounding depends on which of the two its batch takes, as it does between
+// steps and prompts; within a form it does not depend on the batch.
 inline bool step_form_pays(int M, int N, int K, size_t smem) {
   const long long weights = (long long)N * K, most = M <= 8 && K <= 1024 ? 64ll << 20 : M <= 8 && K <= 2048 ? 16ll << 20 : M <= 16 ? 8ll << 20 : 4ll << 20;
-  const int tiles = (N + 15) / 16, most_tiles = M <= 8 ? 0x7fffffff : (M <= 16 ? 2 : 1) * sm_count();
-  return M <= 32 && K <= 4096 && weights <= most && tiles <= most_tiles && smem <= 200 * 1024;
+  const int tiles = (N + 15) / 16, per_sm = M <= 8 ? (K <= 512 ? 4 : 1 << 20) : M <= 16 && K <= 2048 ? 2 : 1;
+  return M <= 32 && K <= 4096 && weights <= most && tiles <= (long long)per_sm * sm_count() && smem <= 200 * 1024;
 }
 
 inline StepGeometry step_geometry(int M, int K) {

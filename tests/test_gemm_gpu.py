@@ -297,3 +297,16 @@ def test_gemm_few_rows_long_k(M, N, K):
     for m in (1, M // 2 + 1):
         assert torch.equal(gemm(x[-m:], w, out_dtype=torch.float32), got[-m:])
     status_ok()
+
+
+# On the far side of the lines: 9 to 16 rows with more tiles than SMs and a K above 2048, up to 8 rows with many tiles of a short K.
+@pytest.mark.parametrize("M,N,K", [(9, 2400, 2304), (16, 2720, 2816), (16, 2560, 3072), (8, 9488, 64), (1, 16384, 256), (8, 32768, 504)])
+def test_gemm_few_rows_in_the_other_form(M, N, K):
+    """These sizes are summed as the ones with 17 or more rows of as many weights are (in the tcgen05 form), bit for bit."""
+    from energonai_b200.gemm import gemm
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, w = torch.randn(32, K, device="cuda", generator=g).half(), (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).half()
+    both = gemm(x, w, out_dtype=torch.float32)
+    assert torch.equal(gemm(x[:M], w, out_dtype=torch.float32), both[:M])
+    check_close(both, reference(x, w), torch.float32)
+    status_ok()
