@@ -436,3 +436,27 @@ def test_gemm_f32_short_k_of_many_columns(N, heads):
             got, plain = per_head(a, w), per_head(odd, w)
             assert torch.equal(got, plain) is not pieces and torch.equal(got[-1:], per_head(a[-1:], w))
             close(got.view(M, heads, N), torch.einsum("mhk,hnk->mhn", a.view(M, heads, K).double(), w.double()), 1e-6)
+
+
+# Prompt rows over a cache: positions from a number on the device, a ring that has wrapped, keys shared by all heads; key rows of every pitch class.
+@pytest.mark.parametrize("dtype", [F32, torch.float16, BF])
+@pytest.mark.parametrize("S,rows,pos,window,dk,dv,shared", [(8, 8, 0, 0, 60, 128, False), (40, 200, 160, 0, 124, 33, True), (33, 70, 500, 30, 92, 64, False),
+                                                            (70, 128, 91, 59, 28, 5, True), (9, 1000, 700, 0, 128, 100, False)])
+def test_plain_attention_in_tiles_of_a_cache(S, rows, pos, window, dk, dv, shared, dtype):
+    """fp32 inside whatever the type: 16-bit results are off by their own rounding, half of 2^-10 or 2^-7."""
+    from energonai_b200.attention import attention_plain
+    B, H, scale = 2, 3, dk ** -0.5
+    G = 1 if shared else H
+    q, k, v = rnd(B, S, H * dk, dtype=dtype), rnd(B, rows, G * dk, seed=1, dtype=dtype), rnd(B, rows, G * dv, seed=2, dtype=dtype)
+    first = torch.tensor([0, pos // 3 if pos < rows else pos - 7], dtype=torch.int32, device="cuda")
+    at = torch.tensor([pos], dtype=torch.int32, device="cuda")
+    got = attention_plain(q, k, v, H, dk, dv, window=window, scale=scale, first=first, pos_device=at, shared_kv=shared)
+    j = torch.arange(max(0, pos + S - rows), pos + S)[None]
+    i = pos + torch.arange(S)[:, None]
+    for b in range(B):
+        seen = (j <= i) & (j >= int(first[b])) & (j > i - (window or rows + S))
+        for h in range(H):
+            g = 0 if shared else h
+            kk, vv = (t[b, j[0] % rows, g * d:(g + 1) * d].double().cpu() for t, d in ((k, dk), (v, dv)))
+            s = (q[b, :, h * dk:(h + 1) * dk].double().cpu() @ kk.T * scale).masked_fill(~seen, -float("inf"))
+            close(got.view(B, S, H, dv)[b, :, h], s.softmax(1) @ vv, {F32: 2e-6, torch.float16: 2 ** -11, BF: 2 ** -8}[dtype])
