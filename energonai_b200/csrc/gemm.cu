@@ -13,7 +13,8 @@
 //       every SM pulls the same number of weight bytes.  A tile shared by several CTAs is
 //       reduced through fp32 partials in a caller-provided workspace by whichever CTA arrives
 //       last, summing in a fixed order, so results are deterministic.
-//   (Prompt-sized products take a tile of 256 rows per pair of SMs, gemm_pair.cuh, where that is faster.  Few rows against a small weight, where a launch's latency is what counts, take gemm_step.cuh instead.)
+//   Prompt-sized products take a tile of 256 rows per pair of SMs, gemm_pair.cuh, where that is faster; few rows
+//   against a small weight, where a launch's latency is what counts, take gemm_step.cuh.
 //
 // Warp roles (192 threads): warp 0 = TMA producer (one lane), warp 1 = TMEM allocation and
 // tcgen05.mma issue (one lane), warps 2-5 = epilogue (tcgen05.ld -> bias / activation /
@@ -37,6 +38,7 @@
 #include "comm.cuh"
 #include "gated.cuh"
 #include "packed_math.cuh"
+#include "weight_stream.cuh"
 #include "xielu.cuh"
 
 namespace eb {
@@ -1596,14 +1598,14 @@ static int gemm_impl(const void *A, long long lda, const void *W, long long ldw,
   p.lane_rows = M; p.col_rows = N;
   const long long lane_tiles = (M + kLanes - 1) / kLanes;
   // Form: the tiles come in waves of one per SM (or pair of SMs); a wave costs its k-blocks and, at its end, an epilogue.  Measured on
-  // products of 64 to 16384 rows, 768 to 20480 columns and K 768 to 20480, microseconds: {columns, one-SM: k-blocks per stage, stages, per
-  // k-block, per wave}; the choice is within 10 % of the best form at all of them.  The narrow pair tile is bound by L2 once most SMs
+  // products of 64 to 16384 rows, 768 to 20480 columns and K 768 to 20480: {rows, columns, k-blocks per stage, stages, us per
+  // k-block, us per wave}; the choice is within 10 % of the best form at all of them.  The narrow pair tile is bound by L2 once most SMs
   // stay busy (0.27).  One-SM tiles stay for few rows (128 x 4096 x 4096: 32 columns 14.0 us, best pair 17.1; 333 x 5120 x 5120: 128 columns
   // 26.0 against 32.4) and lose elsewhere: 8192 x 5120 x 5120 391 us against 299, 12448 x 1024 x 1024 40 against 27, 1024 x 2304 x 768 10.9
-  // against 9.1.  What a row's result is does not depend on the choice.
+  // against 9.1.  What a row's result is does not depend on the choice: each form adds up all of K in one accumulator, in order.
   struct Form { int rows, bn, kpb, stages; float us, wave; };
-  constexpr Form forms[] = {{256, 256, 2, 3, 0.37f, 3.6f}, {256, 128, 2, 4, 0.20f, 1.6f}, {128, 256, 1, 4, 0.45f, 6.f},
-                            {128, 128, 2, 3, 0.28f, 3.2f}, {128, 64, 2, 4, 0.20f, 1.8f},  {128, 32, 3, 3, 0.14f, 1.f}};
+  constexpr Form forms[] = {{256, 256, kPairBlocks, 3, 0.37f, 3.6f}, {256, 128, kPairBlocks, 4, 0.20f, 1.6f}, {128, 256, 1, 4, 0.45f, 6.f},
+                            {128, 128, 2, 3, 0.28f, 3.2f},           {128, 64, 2, 4, 0.20f, 1.8f},            {128, 32, 3, 3, 0.14f, 1.f}};
   Form form = forms[2];
   long long waves = 0;
   if (p.rs) {                                          // (its epilogue turns 64 columns around behind 1-block stages)

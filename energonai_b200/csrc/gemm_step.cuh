@@ -53,19 +53,6 @@ inline StepGeometry step_geometry(int M, int K) {
   return s;
 }
 
-template <typename T> __device__ __forceinline__ void step_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  if (std::is_same<T, __half>::value)
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-  else
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ uint4 step_ld_weight(const void *p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
 // 16 bytes to shared memory, zeros if !ok
 __device__ __forceinline__ void step_cp16(uint32_t dst, const void *src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
@@ -98,8 +85,8 @@ gemm_step_kernel(const GemmParams p, const void *weights, long long ldw, int sli
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const bool ok = live && k0 + u * 32 < ke;
-      w[u][0] = ok ? step_ld_weight(wa + u * 32) : make_uint4(0, 0, 0, 0);
-      w[u][1] = ok ? step_ld_weight(wb + u * 32) : make_uint4(0, 0, 0, 0);
+      w[u][0] = ok ? ld_stream(wa + u * 32) : make_uint4(0, 0, 0, 0);
+      w[u][1] = ok ? ld_stream(wb + u * 32) : make_uint4(0, 0, 0, 0);
     }
     if (++ld_chunk == chunks) { ld_chunk = 0; ld_tile += gridDim.x; }
   };
@@ -245,8 +232,8 @@ gemm_step_kernel(const GemmParams p, const void *weights, long long ldw, int sli
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
           const uint4 x = *reinterpret_cast<const uint4 *>(xk + (size_t)j * 8 * pitch + u * 64);
-          step_mma<T>(acc[j], w[u][0].x, w[u][1].x, w[u][0].y, w[u][1].y, x.x, x.y);
-          step_mma<T>(acc[j], w[u][0].z, w[u][1].z, w[u][0].w, w[u][1].w, x.z, x.w);
+          mma_16816<T>(acc[j], w[u][0].x, w[u][1].x, w[u][0].y, w[u][1].y, x.x, x.y);
+          mma_16816<T>(acc[j], w[u][0].z, w[u][1].z, w[u][0].w, w[u][1].w, x.z, x.w);
           if (fold && first && kb + chunk * 32 * U + u * 32 + t * 8 < p.K) {
             Vec16<T> v;
             v.raw = x;

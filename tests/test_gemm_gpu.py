@@ -310,3 +310,24 @@ def test_gemm_few_rows_in_the_other_form(M, N, K):
     assert torch.equal(gemm(x[:M], w, out_dtype=torch.float32), both[:M])
     check_close(both, reference(x, w), torch.float32)
     status_ok()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_gemm_prompt_forms_agree(dtype):
+    """The same rows in batches that take one-SM tiles of 32, 64, 128 and 256 columns and pair tiles of 128 and 256 with eight and sixteen epilogue
+    warps: bit for bit the same results behind every epilogue, as the choice of a form claims."""
+    from energonai_b200.gemm import gemm, project_unit
+    for N, K, rows in ((1024, 4096, (64, 500, 1000, 2100, 4096, 9000)), (5120, 5120, (64, 333, 600, 777, 4100)), (50272, 768, (40, 130, 520, 1100)), (44912, 168, (65, 300, 900))):
+        g = torch.Generator(device="cuda").manual_seed(N)
+        rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+        w, b = (rnd(N, K) * K ** -0.5).to(dtype), rnd(N).to(dtype)
+        x, res = rnd(max(rows), K).to(dtype), rnd(40, N).to(dtype)
+        want = None
+        for M in rows:
+            a, r = x[:M], torch.zeros(M, N, device="cuda", dtype=dtype)
+            r[:40] = res
+            got = [gemm(a, w)[:40], gemm(a, w, bias=b, act="relu", residual=r)[:40], gemm(a, w, bias=b, act="gelu")[:40], gemm(a, w, bias=b, act="gelu_tanh")[:40],
+                   gemm(a, w, bias=b, out_dtype=torch.float32)[:40], project_unit(a, w, "geglu")[:40]]
+            want = got if want is None else want
+            assert all(torch.equal(p, q) for p, q in zip(got, want)), (N, K, M)
+    status_ok()
