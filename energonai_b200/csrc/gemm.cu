@@ -1599,7 +1599,8 @@ static int gemm_impl(const void *A, long long lda, const void *W, long long ldw,
   const long long lane_tiles = (M + kLanes - 1) / kLanes;
   // Form: the tiles come in waves of one per SM (or pair of SMs); a wave costs its k-blocks and, at its end, an epilogue.  Measured on
   // products of 64 to 16384 rows, 768 to 20480 columns and K 768 to 20480: {rows, columns, k-blocks per stage, stages, us per
-  // k-block, us per wave}; the choice is within 10 % of the best form at all of them.  The narrow pair tile is bound by L2 once most SMs
+  // k-block, us per wave}; the choice is within 5 % of the best form at 95 % of 900 sizes, at worst 19 % off (33 x 3072 x 1024); the
+  // most that it loses to the one-SM tiles alone is 8 % (33 x 50272 x 768, 34 us against 31.5).  The narrow pair tile is bound by L2 once most SMs
   // stay busy (0.27).  One-SM tiles stay for few rows (128 x 4096 x 4096: 32 columns 14.0 us, best pair 17.1; 333 x 5120 x 5120: 128 columns
   // 26.0 against 32.4) and lose elsewhere: 8192 x 5120 x 5120 391 us against 299, 12448 x 1024 x 1024 40 against 27, 1024 x 2304 x 768 10.9
   // against 9.1.  What a row's result is does not depend on the choice: each form adds up all of K in one accumulator, in order.
@@ -1613,6 +1614,7 @@ static int gemm_impl(const void *A, long long lda, const void *W, long long ldw,
   } else {
     float best = 0.f;
     for (const Form &f : forms) {
+      if (f.rows > kLanes && M <= kLanes) continue;    // (the second SM of a pair would have padding: 128 x 8192 x 2048 14.8 us, 64 columns 13.8)
       const long long units = sm_count() * 128 / f.rows, w = ((long long)((M + f.rows - 1) / f.rows) * ((N + f.bn - 1) / f.bn) + units - 1) / units;
       const float us = (float)w * ((float)p.kblocks * (f.rows == 256 && f.bn == 128 && w > 3 ? 0.27f : f.us) + f.wave);
       if (waves == 0 || us < best) { best = us; form = f; waves = w; }
