@@ -272,18 +272,20 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
   if (warp < 4) {
     const int row = warp * 32 + lane, m = m0 + row;
     unsigned long long again = 0;
-    const uint32_t w0 = __float_as_uint(top[kRows + lane]), w1 = __float_as_uint(top[kRows + 32 + lane]);      // (their order is that of the numbers; a NaN above all)
-    const float tw_least = __uint_as_float(__reduce_min_sync(0xffffffffu, min(w0, w1))), tw_most = __uint_as_float(__reduce_max_sync(0xffffffffu, max(w0, w1)));
+    // (Magnitudes are in the order of their bits; a NaN above all.  A row of zeros has exact sums.)
+    const uint32_t w0 = __float_as_uint(top[kRows + lane]), w1 = __float_as_uint(top[kRows + 32 + lane]);
+    const float tw_least = __uint_as_float(__reduce_min_sync(0xffffffffu, min(w0 ? w0 : 0x7f7fffffu, w1 ? w1 : 0x7f7fffffu)));
+    const float tw_most = __uint_as_float(__reduce_max_sync(0xffffffffu, max(w0, w1)));
     if (m < p.M) {
-      // Mostly the whole row is fine by its least and largest sum.
+      // Mostly the whole row is fine by its least and largest sum.  Zeros are, unless every product fell below the range.
       const float ta = top[row], least = (float)p.K * 0x1p-102f;
       float v_least = FLT_MAX, v_most = 0.f;
 #pragma unroll
       for (int j = 0; j < kF32Cols; ++j) {
-        v_least = fminf(v_least, fabsf(acc[j]));
+        v_least = fminf(v_least, acc[j] == 0.f ? FLT_MAX : fabsf(acc[j]));
         v_most = largest(v_most, acc[j], 0.f);
       }
-      if (!(v_most <= FLT_MAX && (ta == 0.f || (fminf(ta, tw_least) >= 0x1p-100f && v_least >= fmaxf(0x1p-100f, least * fmaxf(ta, tw_most)))))) {
+      if (!(v_most <= FLT_MAX && (ta == 0.f || (fminf(fminf(ta, tw_least), ta * tw_least) >= 0x1p-100f && v_least >= fmaxf(0x1p-100f, least * fmaxf(ta, tw_most)))))) {
 #pragma unroll
         for (int j = 0; j < kF32Cols; ++j) {
           const float tw = top[kRows + j], v = fabsf(acc[j]), small = fminf(ta, tw);
@@ -294,6 +296,7 @@ __global__ void __launch_bounds__(kF32TcThreads, 1) gemm_f32_tc_kernel(const F32
       const bool wide = !p.bias && !p.act_params && ((uintptr_t)C & 15) == 0 && p.ldc % 4 == 0;
 #pragma unroll
       for (int j = 0; j < kF32Cols; j += 4) {
+        if (n0 + j >= p.N) break;
         if (wide && n0 + j + 4 <= p.N) {
           *reinterpret_cast<float4 *>(C + (long long)m * p.ldc + n0 + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
         } else {
