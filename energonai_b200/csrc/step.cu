@@ -7,11 +7,11 @@
 // framework kernels is nine launches of a few microseconds each on the critical path of a step
 // that is itself a chain of short launches.
 //
-// A cluster of eight CTAs per sequence: what a step waits for is a row of 200 KB on its way into one SM and, one thread at a time, the trips of
-// its loads (one CTA of 256 threads took 15 to 43 us for 1 to 16 rows of 50272).  Each CTA reads an eighth, leaves its maximum in every other's
-// shared memory, and copies an eighth of the embedding of the token they all arrive at.  The position scalars are read by every CTA before it
-// reports in; the last CTA to report in advances them (so the launches of the next step find them advanced) and
-// rearms the counter.
+// Long rows have a cluster of eight CTAs per sequence: what a step waits for is a row of 200 KB on its way into one SM and, one thread at a time, the
+// trips of its loads (one CTA of 256 threads took 15 to 43 us for 1 to 16 rows of 50272).  Each CTA reads an eighth, leaves its maximum in every
+// other's shared memory, and copies an eighth of the embedding of the token they all arrive at.  Short rows, and so many that they fill the
+// machine by themselves, have one CTA each.  The position scalars are read by every CTA before it reports in; the last
+// CTA to report in advances them (so the launches of the next step find them advanced) and rearms the counter.
 #include <cfloat>
 
 #include "common.cuh"
@@ -19,7 +19,7 @@
 namespace eb {
 namespace {
 
-constexpr int kStepThreads = 256, kStepCtas = 8, kStepWarps = kStepThreads / 32;
+constexpr int kStepThreads = 256, kStepWarps = kStepThreads / 32;
 
 struct StepParams {
   const void *logits;          // [batch][ld_logits], T
@@ -53,12 +53,12 @@ __device__ __forceinline__ uint32_t peer_addr(const void *p, int rank) {
   return r;
 }
 
-// L: type of the logits, T: type of the embedding tables and of the output row
-template <typename L, typename T>
-__global__ void __cluster_dims__(kStepCtas, 1, 1) __launch_bounds__(kStepThreads) greedy_step_kernel(const StepParams p) {
+// L: type of the logits, T: type of the embedding tables and of the output row, kStepCtas: CTAs per sequence
+template <typename L, typename T, int kStepCtas>
+__device__ __forceinline__ void greedy_row(const StepParams &p) {
   __shared__ float s_val[kStepWarps], c_val[kStepCtas];
   __shared__ int s_idx[kStepWarps], c_idx[kStepCtas];
-  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (waited for before another CTA's memory is written)
+  if (kStepCtas > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // (waited for before another CTA's memory is written)
   griddep_wait();
   griddep_launch();
   const int b = blockIdx.x / kStepCtas, rank = blockIdx.x % kStepCtas, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -80,9 +80,12 @@ __global__ void __cluster_dims__(kStepCtas, 1, 1) __launch_bounds__(kStepThreads
     }
   };
   // the row from its first 16-byte boundary on in packs, an eighth of them per CTA; what is left at its ends falls to the first CTA
-  constexpr int VEC = 16 / sizeof(L), kAhead = 4;
+  constexpr int VEC = 16 / sizeof(L), kAhead = kStepCtas > 1 ? 4 : 1;
   const int head = min(p.vocab, (int)((16 - (reinterpret_cast<uintptr_t>(row) & 15u)) % 16 / sizeof(L))), packs = (p.vocab - head) / VEC;
   const int per = (packs + kStepCtas - 1) / kStepCtas, end = min(packs, (rank + 1) * per);
+  const int tail = head + packs * VEC + tid;
+  const bool at_head = rank == 0 && tid < head, at_tail = rank == 0 && tail < p.vocab;
+  const float head_v = at_head ? to_f32<L>(row[tid]) : 0.f, tail_v = at_tail ? to_f32<L>(row[tail]) : 0.f;
   for (int v0 = rank * per + tid; v0 < end; v0 += kAhead * kStepThreads) {
     Vec16<L> pk[kAhead];
 #pragma unroll
@@ -97,26 +100,26 @@ __global__ void __cluster_dims__(kStepCtas, 1, 1) __launch_bounds__(kStepThreads
       for (int e = 0; e < VEC; ++e) take(f[e], head + (v0 + u * kStepThreads) * VEC + e);
     }
   }
-  if (rank == 0) {
-    const int tail = head + packs * VEC + tid;
-    if (tid < head) take(to_f32<L>(row[tid]), tid);
-    if (tail < p.vocab) take(to_f32<L>(row[tail]), tail);
-  }
+  if (at_head) take(head_v, tid);
+  if (at_tail) take(tail_v, tail);
   take_warp();
   if (lane == 0) { s_val[warp] = best; s_idx[warp] = best_i; }
   __syncthreads();
-  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if (kStepCtas > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   if (warp == 0) {
     best = lane < kStepWarps ? s_val[lane] : -FLT_MAX;
     best_i = lane < kStepWarps ? s_idx[lane] : 0x7fffffff;
     take_warp();
-    if (lane < kStepCtas) {
+    if (kStepCtas == 1) {
+      if (lane == 0) { c_val[0] = best; c_idx[0] = best_i; }
+    } else if (lane < kStepCtas) {
       asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_addr(c_val + rank, lane)), "f"(best) : "memory");
       asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(peer_addr(c_idx + rank, lane)), "r"(best_i) : "memory");
     }
     __syncwarp();
   }
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (kStepCtas > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  else __syncthreads();
   best = -FLT_MAX;
   best_i = 0x7fffffff;
 #pragma unroll
@@ -163,17 +166,32 @@ __global__ void __cluster_dims__(kStepCtas, 1, 1) __launch_bounds__(kStepThreads
   }
 }
 
+// (Two kernels: even clusters of one CTA are placed more slowly than CTAs, 4096 of them in 13.6 us instead of 9.)
+template <typename L, typename T> __global__ void __launch_bounds__(kStepThreads) greedy_step_kernel(const StepParams p) { greedy_row<L, T, 1>(p); }
+constexpr int kStepCluster = 8;
+template <typename L, typename T>
+__global__ void __cluster_dims__(kStepCluster, 1, 1) __launch_bounds__(kStepThreads) greedy_step_cluster_kernel(const StepParams p) {
+  greedy_row<L, T, kStepCluster>(p);
+}
+
 }  // namespace
 }  // namespace eb
 
 using namespace eb;
 
 namespace {
+template <typename L, typename T>
+void launch_step_of(int batch, cudaStream_t st, const StepParams &p) {
+  // A cluster costs about 0.5 us, and more with the number of them to place (one row of 50257 9.4 us by one CTA, 3.3 by eight, of 1000 2.3 and 2.6; 128
+  // rows of 50257 10.6 and 8.5, of 8192 3.9 and 6.3; 512 rows of 50257 14.4 and 22.5).
+  if (p.vocab > 6144 + 300 * batch) launch_pdl(greedy_step_cluster_kernel<L, T>, dim3((unsigned)batch * kStepCluster), dim3(kStepThreads), 0, st, p);
+  else launch_pdl(greedy_step_kernel<L, T>, dim3(batch), dim3(kStepThreads), 0, st, p);
+}
 template <typename L>
 void launch_step(int emb_dtype, int batch, cudaStream_t st, const StepParams &p) {
-  if (emb_dtype == EB_F32) launch_pdl(greedy_step_kernel<L, float>, dim3(batch * kStepCtas), dim3(kStepThreads), 0, st, p);
-  else if (emb_dtype == EB_F16) launch_pdl(greedy_step_kernel<L, __half>, dim3(batch * kStepCtas), dim3(kStepThreads), 0, st, p);
-  else launch_pdl(greedy_step_kernel<L, __nv_bfloat16>, dim3(batch * kStepCtas), dim3(kStepThreads), 0, st, p);
+  if (emb_dtype == EB_F32) launch_step_of<L, float>(batch, st, p);
+  else if (emb_dtype == EB_F16) launch_step_of<L, __half>(batch, st, p);
+  else launch_step_of<L, __nv_bfloat16>(batch, st, p);
 }
 }  // namespace
 

@@ -323,3 +323,22 @@ def test_greedy_step_argmax_anywhere(V, dtype):
     greedy_step(logits, out_ids, tok, kv, counter)
     assert tok.tolist() == at + [0, 0] and out_ids[:, 1].tolist() == tok.tolist()
     assert kv.tolist() == [5, 2] and counter.item() == 0
+
+
+@pytest.mark.parametrize("B,V", [(1, 6444), (1, 6445), (3, 9001), (147, 50257), (148, 50257), (300, 2000)])
+def test_greedy_step_rows_and_lengths(B, V):
+    """Both sides of the line between one CTA and a cluster per row: tokens, the embedding of the next position and the advanced positions."""
+    from energonai_b200.step import greedy_step
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = torch.randn(B, V, device="cuda", generator=g).half()
+    want = logits.float().argmax(1)
+    words, positions = torch.randn(V, 72, device="cuda", generator=g).half(), torch.randn(16, 72, device="cuda", generator=g).half()
+    out_ids, tok = torch.full((B, 3), -1, dtype=torch.int64, device="cuda"), torch.empty(B, dtype=torch.int64, device="cuda")
+    kv, counter, hidden = torch.tensor([4, 1], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda"), torch.empty(B, 72, device="cuda").half()
+    for step in range(2):
+        greedy_step(logits, out_ids, tok, kv, counter, word_emb=words, pos_emb=positions, hidden_out=hidden)
+        best = logits.float().max(1).values
+        assert torch.equal(logits.float().gather(1, tok[:, None])[:, 0], best) and torch.equal(out_ids[:, 1 + step], tok)
+        assert torch.equal(hidden, (words[tok].float() + positions[5 + step].float()).half())
+        assert kv.tolist() == [5 + step, 2 + step] and counter.item() == 0
+    assert bool((tok <= want).all())                                  # (the lowest of equal ones)
