@@ -16,6 +16,8 @@
 //   max(first[b], i - window + 1) .. i.
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace eb {
@@ -807,8 +809,16 @@ template <typename T> int launch_tiled(const PlainParams &p, int B, cudaStream_t
 }
 
 template <typename T> int launch_plain(const PlainParams &p, int B, cudaStream_t st) {
-  // Few rows leave most of a tile's rows empty; a cache whose first positions lie in rows of their own is addressed per query.
-  if (p.q_len >= 8 && p.kept_rows == 0 && p.dk % 4 == 0 && p.dk <= kTiledWidth && p.dv <= kTiledWidth) return launch_tiled<T>(p, B, st);
+  // Few rows leave most of a tile's rows empty, and where a row sees few keys its own walk is over before a tile is in place.  The positions that a
+  // row sees at most are held against 16 (rows whose window moves mostly meet two tiles), 8 without window and chunk, and more the narrower the
+  // heads are.  Row by row and by tiles: 64 rows of a head 64 wide, windows of 16 and 32: 16 us and 20, 28 and 23; 8 wide, 16 and 48: 9 and 15, 19
+  // and 17; 64 x 16 heads 64 wide, prompts of 8 and 16: 25 and 36, 61 and 42.  A cache whose first positions lie in rows of their own is addressed per query.
+  long long reach = p.ring_rows;
+  if (p.window > 0) reach = std::min(reach, (long long)p.window + p.keep);
+  if (p.chunk > 0) reach = std::min(reach, (long long)p.chunk + p.keep);
+  const bool pays = p.window > 0 || p.chunk > 0 ? reach * p.dk >= 16 * p.dk + 256 : reach * p.dk >= 8 * p.dk + 192;
+  if (p.q_len >= 8 && pays && p.kept_rows == 0 && p.dk % 4 == 0 && p.dk <= kTiledWidth && p.dv <= kTiledWidth)
+    return launch_tiled<T>(p, B, st);
   int warps = 4;
   const size_t per = (size_t)(p.dk + p.dv) * sizeof(float);
   while (warps > 1 && warps * per > 48 * 1024) warps >>= 1;

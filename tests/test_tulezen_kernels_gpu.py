@@ -460,3 +460,10 @@ def test_plain_attention_in_tiles_of_a_cache(S, rows, pos, window, dk, dv, share
             kk, vv = (t[b, j[0] % rows, g * d:(g + 1) * d].double().cpu() for t, d in ((k, dk), (v, dv)))
             s = (q[b, :, h * dk:(h + 1) * dk].double().cpu() @ kk.T * scale).masked_fill(~seen, -float("inf"))
             close(got.view(B, S, H, dv)[b, :, h], s.softmax(1) @ vv, {F32: 2e-6, torch.float16: 2 ** -11, BF: 2 ** -8}[dtype])
+
+
+# Either side of the line between a warp per row and tiles (positions that a row sees, by head size), and chunks that take tiles.
+@pytest.mark.parametrize("S,dk,dv,rule", [(95, 128, 64, dict(window=17)), (95, 128, 64, dict(window=18)), (200, 64, 33, dict(chunk=19)), (200, 64, 33, dict(chunk=20)),
+                                          (97, 32, 128, dict(chunk=50)), (70, 8, 128, dict(window=40, keep=8, cap=3.0)), (9, 128, 128, dict()), (10, 128, 128, dict()), (31, 8, 8, dict()), (32, 8, 8, dict())])
+def test_plain_attention_by_reach(S, dk, dv, rule):
+    test_plain_attention_in_tiles(S, dk, dv, rule)
