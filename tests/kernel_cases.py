@@ -3,6 +3,7 @@ were taken on, and CUDA-event timings of the kernels that are not part of the be
 
     python tests/kernel_cases.py gemm_decode      # the four OPT-13B generation-step GEMM shapes
     python tests/kernel_cases.py gemm_prefill     # one 8192-row prompt GEMM
+    python tests/kernel_cases.py products         # few rows, true 32-bit, plain attention of a 32-bit prompt
     python tests/kernel_cases.py attention        # prompt (both kernels) and generation-step attention
     python tests/kernel_cases.py attention_speed  # TFLOP/s of the two prompt kernels over sequence lengths
     python tests/kernel_cases.py membound         # event-timed GB/s of the memory-bound kernels
@@ -55,6 +56,27 @@ def gemm_prefill():
         y = gemm(x, w, static_weight=True)
     torch.cuda.synchronize()
     print("gemm_prefill", M, N, K, float((y.float() - x.float() @ w.float().t()).abs().max()))
+
+
+def products():
+    """Each on operands of its own, 200 to 300 MB in all."""
+    from energonai_b200.attention import attention_plain
+    from energonai_b200.gemm import gemm, gemm_f32
+    for M, N, K in ((1, 768, 768), (8, 50257, 768), (16, 2048, 2048), (2, 1024, 4096)):
+        for _ in range(2):
+            w, x = torch.randn(N, K, device="cuda", dtype=torch.float16) * 0.02, torch.randn(M, K, device="cuda", dtype=torch.float16)
+            y = gemm(x, w, static_weight=True)
+        print("few rows", M, N, K, float((y.float() - x.float() @ w.float().t()).abs().max()))
+    for M, N, K in ((333, 11264, 2048), (1, 2048, 2048)):
+        for _ in range(2):
+            w, x = torch.randn(N, K, device="cuda") * 0.02, torch.randn(M, K, device="cuda")
+            y = gemm_f32(x, w)
+        print("32-bit", M, N, K, float((y.double() - x.double() @ w.double().t()).abs().max()))
+    q, k, v = (torch.randn(1, 333, n * 128, device="cuda") for n in (16, 4, 4))
+    for _ in range(2):
+        y = attention_plain(q, k, v, 16, 128, 128, scale=128 ** -0.5, kv_heads=4)
+    torch.cuda.synchronize()
+    print("plain attention", tuple(y.shape))
 
 
 def attention():
@@ -223,5 +245,5 @@ def layernorm():
 
 
 if __name__ == "__main__":
-    {"gemm_decode": gemm_decode, "gemm_prefill": gemm_prefill, "attention": attention, "attention_speed": attention_speed,
+    {"gemm_decode": gemm_decode, "gemm_prefill": gemm_prefill, "products": products, "attention": attention, "attention_speed": attention_speed,
      "membound": membound, "softmax": softmax, "layernorm": layernorm}[sys.argv[1]]()
